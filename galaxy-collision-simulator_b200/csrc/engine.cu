@@ -757,7 +757,8 @@ static int allocate_state(gcs_ctx* c) {
     }
     if (!rc) {
         // worst case: every particle, the most segment-id sort passes
-        c->scratch_cap = scratch_layout(max_segments, capacity, max_segments).end;
+        c->scratch_cap = scratch_layout(max_segments, capacity, max_segments).lookback +
+                         sizeof(uint32_t) * sort_lookback_words_upto(capacity, kKeyPasses + seg_passes(max_segments));
         rc |= dalloc(c, &c->scratch, c->scratch_cap);
     }
     return rc;

@@ -45,9 +45,26 @@ constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
 constexpr int kKeyPasses = 8;          // 63 Morton bits in 8-bit digits
 constexpr int kMaxPasses = 10;         // + up to two segment-id digits
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys per tile
+// Keys per sort tile by the number of pairs (sort_tile): up to kSortSmallMax
+// pairs, one 1024-key tile of 256 threads per SM; above, 512 threads with
+// the fewest keys each (2 to 8) that let all tiles be resident at once, two
+// to an SM, so that a pass is one wave of equal tiles.  Eight passes in CUDA
+// events, 4,096-key tiles for every size before / this rule now: 1,408 pairs
+// 71.7 / 54.2 us, 45,056 91.2 / 70.8, 300,000 104.5 / 89.2, 777,777 150.6 /
+// 124.0, 1,048,576 153.2 / 138.4 (a fixed 4,096-key tile with the new
+// look-back: 777,777 140.3, 1,048,576 140.4).
+constexpr int kSortWave = 2 * 148;
+constexpr int kSortSmallTile = 1024;
+constexpr int64_t kSortSmallMax = 148 * 1024;
+constexpr int kSortThreads = 512;
+constexpr int kSortMaxItems = 8;
+constexpr int kSortTile = kSortThreads * kSortMaxItems;  // the largest tile
+constexpr int sort_tile(int64_t n) {
+    if (n <= kSortSmallMax) return kSortSmallTile;
+    const int64_t items = (n + (int64_t)kSortWave * kSortThreads - 1) / ((int64_t)kSortWave * kSortThreads);
+    return kSortThreads * (int)(items < 2 ? 2 : (items > kSortMaxItems ? kSortMaxItems : items));
+}
+constexpr int kLookGroup = 16;      // tiles per look-back group
 constexpr int kGroupSize = 64;         // walk targets per warp group (two per lane above 32)
 
 // Work unit of the walk: up to kGroupSize consecutive sorted particles of one
@@ -82,7 +99,7 @@ struct Layout {
 //   walk_q    u32[2]                walk work queue          (self-resetting)
 //   bounds    u32[2 * max_segments] ordered min/max          (zeroed by bounds)
 //   tiles     u32[kMaxPasses]       onesweep tile tickets    (zeroed by sort,
-//   lookback  u32[passes][tiles][256] decoupled look-back      with lookback)
+//   lookback  u32[passes][tiles + groups][256] decoupled look-back, with lookback)
 struct ScratchLayout {
     size_t hist, walk_q, bounds, tiles, lookback, end;
 };
@@ -103,6 +120,7 @@ void launch_encode(const Layout& L, const float4* pos, int bounds_mode, float gm
                    int n_seg_passes, cudaStream_t st);
 
 size_t sort_lookback_words(int64_t n, int passes);
+size_t sort_lookback_words_upto(int64_t n, int passes);  // the most any m <= n needs
 void launch_sort_pass(const Layout& L, int pass, const uint64_t* keys_in, const uint32_t* vals_in,
                       uint64_t* keys_out, uint32_t* vals_out, const uint32_t* hist,
                       uint32_t* tile_counter, uint32_t* lookback, uint32_t* status,

@@ -14,7 +14,7 @@
 // Costs and limits of the shared array:
 //   * at most kStaticSortMax (1,048,576) pairs per call; larger sizes are
 //     rejected with GCS_ERR_CAPACITY;
-//   * the array (about 2.1 MB) is held by every GPU that loads this library
+//   * the array (about 2.6 MB) is held by every GPU that loads this library
 //     until the process exits;
 //   * every call uses the same array and leaves its contents behind; each
 //     call clears what must start at zero (histograms, tickets, look-back)
@@ -38,12 +38,18 @@ namespace gcs {
 namespace {
 
 constexpr int64_t kStaticSortMax = int64_t(1) << 20;
-constexpr size_t kStaticTiles = (size_t)((kStaticSortMax + kSortTile - 1) / kSortTile);
 // word offsets inside the array
 constexpr size_t kHistWords = (size_t)kKeyPasses * kRadix;      // digit histograms of all passes
 constexpr size_t kTicketWords = 64;                             // one tile ticket per pass (padded)
 constexpr size_t kStatusWords = 64;                             // fallback status word (padded)
-constexpr size_t kLookbackWords = kStaticTiles * kRadix * kKeyPasses;
+// look-back words: a word per tile and digit and one per look-back group and
+// digit, for one full wave of tiles (calls of up to kStaticSortMax pairs)
+constexpr size_t kStaticTiles = kSortWave;
+static_assert((kStaticSortMax + sort_tile(kStaticSortMax) - 1) / sort_tile(kStaticSortMax) <= kSortWave &&
+                  kSortSmallMax / kSortSmallTile <= kSortWave,
+              "every call's tiles fit the array");
+constexpr size_t kStaticSlots = kStaticTiles + (kStaticTiles + kLookGroup - 1) / kLookGroup;
+constexpr size_t kLookbackWords = kStaticSlots * kRadix * kKeyPasses;
 constexpr size_t kScratchWords = kHistWords + kTicketWords + kStatusWords + kLookbackWords;
 
 }  // namespace
@@ -116,8 +122,7 @@ extern "C" int gcs_sort_pairs_static(uint64_t* keys, uint32_t* vals, uint64_t* k
     uint32_t* tickets = base + kHistWords;
     uint32_t* own_status = tickets + kTicketWords;
     uint32_t* lookback = own_status + kStatusWords;
-    const int64_t tiles = (n + kSortTile - 1) / kSortTile;
-    const size_t clear_words = kHistWords + kTicketWords + kStatusWords + (size_t)tiles * kRadix * kKeyPasses;
+    const size_t clear_words = kHistWords + kTicketWords + kStatusWords + sort_lookback_words(n, kKeyPasses);
     if (cudaMemsetAsync(base, 0, clear_words * sizeof(uint32_t), st) != cudaSuccess) return GCS_ERR_CUDA;
     int64_t grid = (n + 255) / 256;
     const int64_t cap = (int64_t)current_sm_count() * 8;  // 8 resident 256-thread blocks per SM

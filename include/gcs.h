@@ -351,7 +351,7 @@ int gcs_autotune(gcs_ctx* ctx, gcs_params* p, double* best_walk_ms);
  * call only queues work on `stream`.  With status == NULL the call waits for
  * `stream` and returns GCS_ERR_DEVICE if a pass gave up.  The
  * histograms and look-back state live in one static device array of about
- * 2.1 MB that every GPU loading this library keeps until exit; no call
+ * 2.6 MB that every GPU loading this library keeps until exit; no call
  * allocates.  Each call clears that array on `stream` (a cudaStream_t, NULL
  * = legacy default) before using it, so calls ordered on the GPU are
  * independent, but calls that overlap on the GPU race on it.  The first
