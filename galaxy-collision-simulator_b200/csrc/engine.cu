@@ -56,6 +56,7 @@ struct gcs_ctx {
     // or leaf size, first rewrites them from the traverse records.
     WalkNode* wn = nullptr;
     uint64_t tree_gen = 1;
+    bool relay_empty = false;  // a build was queued since the last aggregation (launch_relay_reset)
     uint64_t wn_gen = 0;
     float wn_G = 0.0f;
     int32_t wn_L = 0;
@@ -200,6 +201,7 @@ ScratchLayout scratch_layout(int32_t max_segments, int64_t n, int nseg) {
     ScratchLayout s;
     s.hist = 0;
     s.walk_q = round256(sizeof(uint32_t) * kMaxPasses * kRadix);
+    s.agg_q = s.walk_q + 128;
     s.bounds = s.walk_q + 256;
     s.tiles = s.bounds + round256(sizeof(uint32_t) * 2 * (size_t)max_segments);
     s.lookback = s.tiles + 256;
@@ -572,7 +574,10 @@ static int run_stage(gcs_ctx* c, const gcs_params* p, int stage, bool gather_bes
             return check_launch(c, "gather");
         }
         case GCS_STAGE_BUILD:
-            launch_build(L, c->keys[c->sorted_buf], c->tr, c->bd, c->leaf_parent, c->status, st);
+            launch_build(L, c->keys[c->sorted_buf], c->tr, c->bd, c->leaf_parent, c->wn, c->com64,
+                         scratch_at<uint32_t>(c, sl.agg_q), c->status, st);
+            c->relay_empty = true;
+            c->tree_gen++;  // the walk records of the nodes above the blocks are gone
             if (c->gather_pending) {  // later stages read the gathered records
                 GCS_CUDA(c, cudaStreamWaitEvent(st, c->gather_join, 0));
                 c->gather_pending = false;
@@ -580,7 +585,11 @@ static int run_stage(gcs_ctx* c, const gcs_params* p, int stage, bool gather_bes
             return check_launch(c, "build");
         case GCS_STAGE_AGGREGATE: {
             const WalkNodeParams wnp = walk_node_params(c, p);
+            uint32_t* ticket = scratch_at<uint32_t>(c, sl.agg_q);
+            if (!c->relay_empty) launch_relay_reset(L, c->tr, c->wn, c->com64, ticket, st);
+            c->relay_empty = false;
             launch_aggregate(L, c->pos[c->cur], c->tr, c->bd, c->com64, c->leaf_parent, p->com_fp64, wnp,
+                             reinterpret_cast<int2*>(c->keys[c->sorted_buf ^ 1]), c->idx[c->sorted_buf ^ 1], ticket,
                              c->status, st);
             c->tree_gen++;
             c->wn_gen = c->tree_gen;
@@ -1123,6 +1132,7 @@ int gcs_step(gcs_ctx* c, const gcs_params* p) {
     GCS_CUDA(c, cudaGraphLaunch(c->graph_exec[c->cur], c->stream));
     c->cur = c->graph_after[c->cur];  // the flips the captured step made (gather, kick/drift in the walk)
     c->sorted_buf = (kKeyPasses + seg_passes(c->nseg)) & 1;
+    c->relay_empty = false;  // the captured aggregation used it
     return GCS_OK;
 }
 

@@ -102,11 +102,12 @@ struct Layout {
 // region it accumulates into, so any stage can be run on its own:
 //   hist      u32[kMaxPasses][256]  radix digit histograms   (zeroed by encode)
 //   walk_q    u32[2]                walk work queue          (self-resetting)
+//   agg_q     u32                   aggregation block ticket (zeroed by build)
 //   bounds    u32[2 * max_segments] ordered min/max          (zeroed by bounds)
 //   tiles     u32[kMaxPasses]       onesweep tile tickets    (zeroed by sort,
 //   lookback  u32[passes][tiles + groups][256] decoupled look-back, with lookback)
 struct ScratchLayout {
-    size_t hist, walk_q, bounds, tiles, lookback, end;
+    size_t hist, walk_q, agg_q, bounds, tiles, lookback, end;
 };
 
 // ---- launchers (one per stage; all asynchronous on `st`) ----------------
@@ -133,12 +134,21 @@ void launch_sort_pass(const Layout& L, int pass, const uint64_t* keys_in, const 
 
 void launch_gather(const uint32_t* idx, const float4* pos_in, const float4* vel_in, float4* pos_out,
                    float4* vel_out, int64_t n, cudaStream_t st);
-void launch_build(const Layout& L, const uint64_t* keys, BvhNodeTraverse* tr, BvhNodeBuild* bd,
-                  int32_t* leaf_parent, uint32_t* status, cudaStream_t st);
+struct WalkNode;
 struct WalkNodeParams;
+// The build also empties the aggregation's relay (k_tree.cu: words of wn, tr
+// and com64 of the nodes above its blocks) and zeroes its block ticket; an
+// aggregation that does not follow a build needs launch_relay_reset first.
+// roots, n_roots: the aggregation's lists between its two launches, n records
+// each (the sort's spare key and index buffers).
+void launch_build(const Layout& L, const uint64_t* keys, BvhNodeTraverse* tr, BvhNodeBuild* bd,
+                  int32_t* leaf_parent, WalkNode* wn, double4* com64, uint32_t* agg_ticket, uint32_t* status,
+                  cudaStream_t st);
+void launch_relay_reset(const Layout& L, BvhNodeTraverse* tr, WalkNode* wn, double4* com64, uint32_t* agg_ticket,
+                        cudaStream_t st);
 void launch_aggregate(const Layout& L, const float4* pos, BvhNodeTraverse* tr, BvhNodeBuild* bd,
                       double4* com64, const int32_t* leaf_parent, int com_fp64, const WalkNodeParams& wnp,
-                      uint32_t* status, cudaStream_t st);
+                      int2* roots, uint32_t* n_roots, uint32_t* agg_ticket, uint32_t* status, cudaStream_t st);
 
 struct WalkParams {
     float G, eps2, theta2;
@@ -165,7 +175,7 @@ struct WalkNode {
 static_assert(sizeof(WalkNode) == 32, "WalkNode must be 32 bytes");
 constexpr int kWalkBucketTag = 1 << 30;
 constexpr int kWalkSkipTag = 0x7FFFFFFF;
-// G and leaf size of the walk records an aggregation writes (wn null: none).
+// G and leaf size of the walk records an aggregation writes.
 struct WalkNodeParams {
     WalkNode* wn;
     float G;

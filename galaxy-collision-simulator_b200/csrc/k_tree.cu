@@ -12,15 +12,15 @@
 // builds for that segment alone.  Each node also records the far end of its
 // particle range, which gives the walk the node's particle count.
 //
-// Aggregation: a climb starts at every particle's leaf (a lane runs one climb
-// after another over its block's particles); at each node the first arrival
-// stops and the second computes the node from both children
-// (karras_bvh.cuh:175-225).  Unlike the reference, the arrival counter is a
-// release/acquire handshake (__threadfence on both sides and L2-coherent
-// loads of the children), so the second arrival always sees the first one's
-// writes.  Centres of mass are either the reference's FP32 formula or FP64
-// mass-weighted sums carried up the tree (exact for leaf terms, no
-// cancellation at the top of the tree), rounded once to FP32.
+// Aggregation: a climb starts at every particle's leaf and goes up as long as
+// both children of a node are known (karras_bvh.cuh:175-225).  Nodes inside a
+// block's run of particles are climbed in shared memory; above them the left
+// child's values are handed to the right child's climber through global
+// memory word by word (the relay below), so, unlike in the reference, a node
+// is never computed from values its children have not written.  Centres of
+// mass are either the reference's FP32 formula or FP64 mass-weighted sums
+// carried up the tree (exact for leaf terms, no cancellation at the top of
+// the tree), rounded once to FP32.
 #include "gcs_internal.h"
 #include "device_math.cuh"
 
@@ -28,20 +28,69 @@ namespace gcs {
 
 namespace {
 
-// Arrival counter increment with acquire-release semantics at GPU scope.
-__device__ __forceinline__ int arrive_acq_rel(int32_t* flag) {
-    int old;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(flag) : "memory");
-    return old;
+constexpr int kAggThreads = 128;     // threads of an aggregation block
+constexpr int kAggRange = 256;       // particles a block owns (measured at aggregate_kernel)
+constexpr uint32_t kRelayPolls = 1u << 22;  // turns a climber waits for its left child (seconds)
+constexpr int kAggMaxLevels = 96;    // internal levels of a valid tree (strictly increasing prefix lengths)
+
+// ---- relay ------------------------------------------------------------------
+// A node whose particles lie in more than one block's run (aggregate_kernel)
+// is computed by its right child's climber, which gets the left child's
+// values from the node's own records, before they hold the node's values:
+//   wn     lo.x lo.y lo.z hi.x | hi.y hi.z com.x com.y     (32-bit words)
+//   tr     com.z mass
+//   com64  the FP64 sums, of a left child that has them    (64-bit words)
+// The build (or launch_relay_reset) sets every word of these to all ones, the
+// left child's climber writes them, and a word that is not all ones is there:
+// each is a single relaxed access and needs no fence, counter or order among
+// the others.  All ones is a NaN no arithmetic gives; a value with those bits
+// (a NaN position of the caller's) is handed on as another NaN.
+__device__ __forceinline__ uint4 load_relaxed(const void* p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
 }
-__device__ __forceinline__ int arrive_relaxed(int32_t* flag) {
-    int old;
-    asm volatile("atom.relaxed.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(flag) : "memory");
-    return old;
+__device__ __forceinline__ uint2 load_relaxed2(const void* p) {
+    uint2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    return v;
 }
-// Acquire side of a relaxed arrival (the fence makes the sibling's writes,
-// released by its own acq_rel arrival, visible to the loads that follow).
-__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ ulonglong2 load_relaxed64(const void* p) {
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_relaxed(uint4* p, uint4 v) {
+    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};"
+                 :: "l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void store_relaxed(uint2* p, uint2 v) {
+    asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" :: "l"(p), "r"(v.x), "r"(v.y) : "memory");
+}
+__device__ __forceinline__ void store_relaxed(ulonglong2* p, ulonglong2 v) {
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" :: "l"(p), "l"(v.x), "l"(v.y) : "memory");
+}
+__device__ __forceinline__ uint32_t relay_word(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return u == 0xFFFFFFFFu ? 0x7FFFFFFFu : u;
+}
+__device__ __forceinline__ unsigned long long relay_word(double f) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(f);
+    return u == ~0ull ? 0x7FFFFFFFFFFFFFFFull : u;
+}
+__device__ __forceinline__ void relay_clear(WalkNode* wn, BvhNodeTraverse* tr, double4* com64, int node) {
+    const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+    uint4* w = reinterpret_cast<uint4*>(wn + node);
+    w[0] = ones;
+    w[1] = ones;
+    *reinterpret_cast<uint2*>(tr + node) = make_uint2(~0u, ~0u);
+    uint4* q = reinterpret_cast<uint4*>(com64 + node);
+    q[0] = ones;
+    q[1] = ones;
+}
+// Whether particles [lo, hi] lie in more than one aggregation block's run.
+__device__ __forceinline__ bool above_blocks(int lo, int hi) { return lo / kAggRange != hi / kAggRange; }
 
 // Common prefix length of sorted keys i and j of one segment (local indices);
 // -1 when j falls outside the segment.
@@ -55,7 +104,10 @@ __device__ __forceinline__ int lcp(int i, int j, int n, const uint64_t* __restri
 
 __global__ void build_kernel(Layout L, const uint64_t* __restrict__ keys,
                              BvhNodeTraverse* __restrict__ tr, BvhNodeBuild* __restrict__ bd,
-                             int32_t* __restrict__ leaf_parent, uint32_t* __restrict__ status) {
+                             int32_t* __restrict__ leaf_parent, WalkNode* __restrict__ wn,
+                             double4* __restrict__ com64, uint32_t* __restrict__ agg_ticket,
+                             uint32_t* __restrict__ status) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *agg_ticket = 0u;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < L.n; g += gridDim.x * blockDim.x) {
         const int s = L.nseg > 1 ? __ldg(L.seg_id + g) : 0;
         const int off = (int)__ldg(L.seg_off + s);
@@ -103,6 +155,7 @@ __global__ void build_kernel(Layout L, const uint64_t* __restrict__ keys,
         else bd[cr].parent = node;
         bd[node].flag = 0;
         if (i == 0) bd[node].parent = -1;       // segment root
+        if (above_blocks(off + lo, off + hi)) relay_clear(wn, tr, com64, node);
     }
 }
 
@@ -113,40 +166,6 @@ struct ChildData {
     double md;    // FP64 mass sum
 };
 
-// Loads child c; its FP64 sums only when `fp64` (the caller's test that c is
-// an internal node of at least kComFp64Min particles under a node that sums
-// in FP64; a particle is never one).
-__device__ __forceinline__ ChildData load_child(int c, int n_internal, const float4* __restrict__ pos,
-                                                const BvhNodeTraverse* tr, const BvhNodeBuild* bd,
-                                                const double4* com64, bool fp64) {
-    ChildData r;
-    if (c >= n_internal) {
-        const float4 p = __ldg(pos + (c - n_internal));
-        r.lo = r.hi = r.com = make_float3(p.x, p.y, p.z);
-        r.m = p.w;
-    } else {
-        // Written by another thread of this launch: read through L2.
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(tr + c));
-        const float4 b0 = __ldcg(reinterpret_cast<const float4*>(bd + c));
-        const float2 b1 = __ldcg(reinterpret_cast<const float2*>(bd + c) + 2);
-        r.com = make_float3(a.x, a.y, a.z);
-        r.m = a.w;
-        r.lo = make_float3(b0.x, b0.y, b0.z);
-        r.hi = make_float3(b0.w, b1.x, b1.y);
-        if (fp64) {
-            const double2 q0 = __ldcg(reinterpret_cast<const double2*>(com64 + c));
-            const double2 q1 = __ldcg(reinterpret_cast<const double2*>(com64 + c) + 1);
-            r.mx = make_double3(q0.x, q0.y, q1.x);
-            r.md = q1.y;
-        }
-    }
-    return r;
-}
-
-constexpr uint32_t kFull = 0xFFFFFFFFu;
-constexpr int kAggThreads = 128;     // threads of an aggregation block
-constexpr int kAggRange = 512;       // particles a block owns (its lanes take them as they finish)
-constexpr int kAggBlocksPerSm = 8;
 // FP64 centre-of-mass sums (com_fp64) are kept for the top of the tree:
 // nodes of at least this many particles, where the mass-weighted positions
 // of many particles are summed.  A child below the size (or a particle)
@@ -155,21 +174,6 @@ constexpr int kAggBlocksPerSm = 8;
 // particles, so they are never FP64 nodes.
 constexpr int kComFp64Min = 1024;
 static_assert(kComFp64Min > kAggRange, "block-local nodes are never FP64 nodes");
-
-// A node finished inside the block, kept in shared memory for its parent.
-struct LocalNode {
-    float3 lo, hi, com;
-    float m;
-};
-
-__device__ __forceinline__ ChildData from_local(const LocalNode& q) {
-    ChildData r;
-    r.lo = q.lo;
-    r.hi = q.hi;
-    r.com = q.com;
-    r.m = q.m;
-    return r;
-}
 
 // A child's terms in its parent's FP64 sums: its own sums if it is an FP64
 // node, else the double product of its FP32 mass and centre of mass.
@@ -231,193 +235,383 @@ __global__ void walk_nodes_kernel(Layout L, const BvhNodeTraverse* __restrict__ 
     }
 }
 
-// Block b owns particles [kAggRange b, kAggRange (b + 1)).  A node whose
-// particle range lies inside its block's range has both children finished by
-// threads of that block: its arrival counter and the finished children live
-// in shared memory and the handshake is block-scoped.  Every other node uses
-// the GPU-scope counter in its build record.  The side a node uses depends
-// only on the node, so both arrivals always meet.
+// A node's own values from its two children's: box, width, mass, and the
+// centre of mass in the reference's FP32 formula (of FP64 nodes the caller
+// replaces it).
+__device__ __forceinline__ float merge_children(const ChildData& A, const ChildData& B, ChildData& out) {
+    out.lo = make_float3(fminf(A.lo.x, B.lo.x), fminf(A.lo.y, B.lo.y), fminf(A.lo.z, B.lo.z));
+    out.hi = make_float3(fmaxf(A.hi.x, B.hi.x), fmaxf(A.hi.y, B.hi.y), fmaxf(A.hi.z, B.hi.z));
+    out.m = __fadd_rn(A.m, B.m);
+    return fmaxf(__fsub_rn(out.hi.x, out.lo.x),
+                 fmaxf(__fsub_rn(out.hi.y, out.lo.y), __fsub_rn(out.hi.z, out.lo.z)));
+}
+__device__ __forceinline__ float3 merged_com_fp32(const ChildData& A, const ChildData& B, const ChildData& n) {
+    if (n.m > 0.0f)
+        return make_float3(com_fp32(A.com.x, A.m, B.com.x, B.m, n.m), com_fp32(A.com.y, A.m, B.com.y, B.m, n.m),
+                           com_fp32(A.com.z, A.m, B.com.z, B.m, n.m));
+    return make_float3(__fmul_rn(__fadd_rn(n.lo.x, n.hi.x), 0.5f), __fmul_rn(__fadd_rn(n.lo.y, n.hi.y), 0.5f),
+                       __fmul_rn(__fadd_rn(n.lo.z, n.hi.z), 0.5f));
+}
+
+// A block's nodes in shared memory, by the particle at the node's own end of
+// its range (slot 0 is the block's first particle).
+struct AggSmem {
+    float4 pos[kAggRange];        // the particles
+    int4 link[kAggRange];         // children, far end of the range, parent (-2: not a node of this block)
+    float4 com_m[kAggRange];      // finished nodes
+    float4 box_a[kAggRange];      // min x y z, max x
+    float2 box_b[kAggRange];      // max y z
+    int32_t arrived[kAggRange];
+    uint16_t queue[3][kAggRange / 2 + 1];  // nodes whose children are both finished, by step
+    int n_queue[3];
+    int n_roots;                  // finished subtrees whose parent lies above the block
+};
+constexpr int kNotLocal = -2;
+
+__device__ __forceinline__ ChildData smem_particle(const AggSmem& S, int slot) {
+    ChildData r;
+    const float4 p = S.pos[slot];
+    r.lo = r.hi = r.com = make_float3(p.x, p.y, p.z);
+    r.m = p.w;
+    return r;
+}
+__device__ __forceinline__ ChildData smem_node(const AggSmem& S, int slot) {
+    ChildData r;
+    const float4 c = S.com_m[slot], a = S.box_a[slot];
+    const float2 b = S.box_b[slot];
+    r.com = make_float3(c.x, c.y, c.z);
+    r.m = c.w;
+    r.lo = make_float3(a.x, a.y, a.z);
+    r.hi = make_float3(a.w, b.x, b.y);
+    return r;
+}
+
+// Block b owns particles [kAggRange b, kAggRange (b + 1)).  A node is local
+// to the block when its whole particle range lies inside; both children are
+// then finished by this block.
 //
-// Each lane climbs from one particle at a time: it arrives at the parent of
-// what it has just finished; the first arrival stops, the second computes the
-// parent and climbs on.  A lane whose climb has stopped takes the block's
-// next particle at once (the warp claims particles for all its idle lanes
-// with one shared-memory atomic), so a warp keeps its lanes busy instead of
-// running as long as its longest-climbing lane.  Which lane computes a node
-// does not change its value.
-__global__ void __launch_bounds__(kAggThreads, kAggBlocksPerSm)
+//   load    the block's particles, leaf parents and node links, coalesced;
+//   climb   local nodes, in shared memory alone, in block-wide steps: each
+//           step computes the nodes whose two children are finished, packed
+//           into whole warps (a step waits on no global load, store or
+//           fence, and a climb by every particle's own lane keeps 8 lanes of
+//           a warp busy).  A subtree whose parent is not local is left on a
+//           list;
+//   store   the finished nodes' records, whole and coalesced.
+// The nodes above the blocks are rise_kernel's.
+__global__ void __launch_bounds__(kAggThreads)
 aggregate_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restrict__ tr,
-                 BvhNodeBuild* __restrict__ bd, double4* __restrict__ com64,
-                 const int32_t* __restrict__ leaf_parent, int com_fp64, WalkNodeParams wnp,
-                 uint32_t* __restrict__ status) {
-    __shared__ int sflag[kAggRange];
-    __shared__ LocalNode snode[kAggRange];
-    __shared__ int s_next;  // the block's next unclaimed particle
-    const bool fp64 = com_fp64 != 0;
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt = (1u << lane) - 1u;
+                 BvhNodeBuild* __restrict__ bd, const int32_t* __restrict__ leaf_parent, WalkNodeParams wnp,
+                 int2* __restrict__ roots, uint32_t* __restrict__ n_roots, uint32_t* __restrict__ status) {
+    __shared__ AggSmem S;
     const int ni = L.n_internal;
+    const int lim = ni + L.n;
+    if (threadIdx.x == 0) {
+        S.n_roots = 0;
+        S.n_queue[0] = S.n_queue[1] = S.n_queue[2] = 0;
+    }
     const int b0 = blockIdx.x * kAggRange;
-    const int b_end = min(b0 + kAggRange, L.n);
-    for (int i = threadIdx.x; i < kAggRange; i += kAggThreads) sflag[i] = 0;
-    if (threadIdx.x == 0) s_next = b0;
-    __syncthreads();
-    bool have = false;  // this lane is climbing
-    int s = 0, seg_lo = 0, seg_hi = 0, from = 0, node = -1, cl = -1, cr = -1, up = -1, re = 0, levels = 0;
-    ChildData mine;
-    for (;;) {
-        // idle lanes take the block's next particles
-        const uint32_t idle = __ballot_sync(kFull, !have);
-        if (idle) {
-            const int leader = __ffs(idle) - 1;
-            int base = 0;
-            if (lane == leader) base = atomicAdd(&s_next, __popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            if (!have) {
-                const int g = base + __popc(idle & lt);
-                if (g < b_end) {
-                    s = L.nseg > 1 ? __ldg(L.seg_id + g) : 0;
-                    seg_lo = (int)__ldg(L.seg_off + s);
-                    seg_hi = (int)__ldg(L.seg_off + s + 1) - 1;
-                    from = ni + g;
-                    mine = load_child(from, ni, pos, tr, bd, com64, false);
-                    node = __ldg(leaf_parent + g);
-                    levels = 0;
-                    if (node >= 0 && node < ni) {
-                        cl = __ldg(&tr[node].child_left);
-                        cr = __ldg(&tr[node].child_right);
-                        up = __ldg(&bd[node].parent);
-                        re = __ldg(&tr[node].range_end);
-                    }
-                    have = node >= 0;  // a one-particle segment has no parent
-                }
+    const int count = min(kAggRange, L.n - b0);
+    const auto seg_of = [&](int g) { return L.nseg > 1 ? (int)__ldg(L.seg_id + g) : 0; };
+    const auto seg_end = [&](int s) { return L.nseg > 1 ? (int)__ldg(L.seg_off + s + 1) : L.n; };
+
+    // ---- load
+    int my_parent[kAggRange / kAggThreads];  // of the thread's particles
+#pragma unroll
+    for (int u = 0; u < kAggRange / kAggThreads; ++u) {
+        const int j = threadIdx.x + u * kAggThreads;
+        my_parent[u] = -1;
+        if (j >= count) break;
+        const int g = b0 + j, s = seg_of(g);
+        S.pos[j] = __ldg(pos + g);
+        my_parent[u] = __ldg(leaf_parent + g);
+        S.arrived[j] = 0;
+        int4 k = make_int4(-1, -1, 0, kNotLocal);
+        if (g + 1 < seg_end(s)) {  // node g - s exists
+            const int node = g - s;
+            const int4 t = __ldg(reinterpret_cast<const int4*>(tr + node) + 1);  // width, left, right, range end
+            const int up = __ldg(&bd[node].parent);
+            const int lo = min(g, t.w), hi = max(g, t.w);
+            if (lo >= b0 && hi < b0 + count) {
+                if (t.y < 0 || t.z < 0 || t.y >= lim || t.z >= lim) atomicOr(status, GCS_DEV_TREE_MALFORMED);
+                else k = make_int4(t.y, t.z, t.w, up);
             }
         }
-        if (!__any_sync(kFull, have)) break;
-        if (!have) continue;
-        // one step of this lane's climb: arrive at `node`, the parent of `from`
-        // (a valid tree has at most 96 internal levels: strictly increasing
-        // prefix lengths below 96; more means malformed parent links)
-        if (++levels > 96 || node >= ni) {
-            atomicOr(status, GCS_DEV_TREE_MALFORMED);
-            have = false;
-            continue;
+        S.link[j] = k;
+    }
+    __syncthreads();
+
+    // ---- climb
+    // arrive: `from` is finished; the second child to arrive at a local parent
+    // queues it for the next step, a subtree under any other parent is a root
+    const auto arrive = [&](int from, int up, int sg, int q) {
+        if (up < 0) return;  // the segment's root (or a one-particle segment)
+        const int slot = up + sg - b0;
+        if (slot < 0 || slot >= count || S.link[slot].w == kNotLocal) {
+            roots[b0 + atomicAdd(&S.n_roots, 1)] = make_int2(from, sg);
+        } else if (atomicAdd(&S.arrived[slot], 1) == 1) {
+            S.queue[q][atomicAdd(&S.n_queue[q], 1)] = (uint16_t)slot;
         }
-        const int own = node + s;  // particle index at this end of the node's range
-        const bool local = min(own, re) >= b0 && max(own, re) < b0 + kAggRange;
-        int old;
-        if (local) {
-            // block scope: this lane's writes (shared and global) before the
-            // arrival, the sibling's after it
-            __threadfence_block();
-            old = atomicAdd(&sflag[own - b0], 1);
-            if (old != 0) __threadfence_block();
-        } else if (levels == 1) {
-            // at the leaf level this lane has written nothing for `from`, so
-            // its arrival needs no release; it acquires only if it arrives second
-            old = arrive_relaxed(&bd[node].flag);
-            if (old != 0) fence_acq_rel();
-        } else {
-            // release: the child this lane just finished is visible to whoever
-            // acquires the counter next; acquire: the second arrival sees the
-            // sibling's writes
-            old = arrive_acq_rel(&bd[node].flag);
-        }
-        if (old == 0) {  // first arrival: the sibling's climb finishes the node
-            have = false;
-            continue;
-        }
-        if (cl < 0 || cr < 0 || cl >= ni + L.n || cr >= ni + L.n || (cl != from && cr != from)) {
-            atomicOr(status, GCS_DEV_TREE_MALFORMED);
-            have = false;
-            continue;
-        }
-        int ncl = -1, ncr = -1, nup = -1, nre = 0;
-        if (up >= 0 && up < ni) {
-            ncl = __ldg(&tr[up].child_left);
-            ncr = __ldg(&tr[up].child_right);
-            nup = __ldg(&bd[up].parent);
-            nre = __ldg(&tr[up].range_end);
-        }
-        const bool left = cl == from;
-        const int sib = left ? cr : cl;
-        // particles of the node and of its two children (the split is the
-        // left child's end of the range)
-        const int lo_p = min(own, re), hi_p = max(own, re);
-        const int split = cl >= ni ? cl - ni : cl + s;
-        const bool big = fp64 && hi_p - lo_p + 1 >= kComFp64Min;
-        const bool big_l = big && split - lo_p + 1 >= kComFp64Min;
-        const bool big_r = big && hi_p - split >= kComFp64Min;
-        // a local node's internal children are local too: read them from
-        // shared memory (their own range end is inside the block)
-        ChildData other;
-        if (local && sib < ni) {
-            const int so = sib + s - b0;
-            if (so < 0 || so >= kAggRange) {
+    };
+#pragma unroll
+    for (int u = 0; u < kAggRange / kAggThreads; ++u) {
+        const int j = threadIdx.x + u * kAggThreads;
+        if (j < count) arrive(ni + b0 + j, my_parent[u], seg_of(b0 + j), 0);
+    }
+    __syncthreads();
+    for (int step = 0; S.n_queue[step % 3] > 0; ++step) {
+        const int q = step % 3, n_ready = S.n_queue[q];
+        if (threadIdx.x == 0) S.n_queue[(step + 2) % 3] = 0;
+        for (int e = threadIdx.x; e < n_ready; e += kAggThreads) {
+            const int slot = S.queue[q][e];
+            const int4 k = S.link[slot];
+            const int sg = seg_of(b0 + slot);
+            const int sl = k.x >= ni ? k.x - ni - b0 : k.x + sg - b0, sr = k.y >= ni ? k.y - ni - b0 : k.y + sg - b0;
+            if (sl < 0 || sr < 0 || sl >= count || sr >= count) {
                 atomicOr(status, GCS_DEV_TREE_MALFORMED);
-                have = false;
                 continue;
             }
-            other = from_local(snode[so]);
-        } else {
-            other = load_child(sib, ni, pos, tr, bd, com64, left ? big_r : big_l);
+            const ChildData A = k.x >= ni ? smem_particle(S, sl) : smem_node(S, sl);
+            const ChildData B = k.y >= ni ? smem_particle(S, sr) : smem_node(S, sr);
+            ChildData node;
+            merge_children(A, B, node);
+            node.com = merged_com_fp32(A, B, node);
+            S.com_m[slot] = make_float4(node.com.x, node.com.y, node.com.z, node.m);
+            S.box_a[slot] = make_float4(node.lo.x, node.lo.y, node.lo.z, node.hi.x);
+            S.box_b[slot] = make_float2(node.hi.y, node.hi.z);
+            arrive(b0 + slot - sg, k.w, sg, (step + 1) % 3);
         }
-        const ChildData& A = left ? mine : other;   // left child
-        const ChildData& B = left ? other : mine;   // right child
-        const float3 lo = make_float3(fminf(A.lo.x, B.lo.x), fminf(A.lo.y, B.lo.y), fminf(A.lo.z, B.lo.z));
-        const float3 hi = make_float3(fmaxf(A.hi.x, B.hi.x), fmaxf(A.hi.y, B.hi.y), fmaxf(A.hi.z, B.hi.z));
-        const float width = fmaxf(__fsub_rn(hi.x, lo.x), fmaxf(__fsub_rn(hi.y, lo.y), __fsub_rn(hi.z, lo.z)));
-        const float m = __fadd_rn(A.m, B.m);
-        float3 com;
-        ChildData next;
-        next.md = 0.0;
-        next.mx = make_double3(0.0, 0.0, 0.0);
-        if (m > 0.0f) {
-            if (big) {
+        __syncthreads();
+    }
+
+    // ---- store
+    for (int j = threadIdx.x; j < count; j += kAggThreads) {
+        const int4 k = S.link[j];
+        if (k.w == kNotLocal || S.arrived[j] < 2) continue;
+        const int g = b0 + j, s = seg_of(g), node = g - s;
+        const float4 c = S.com_m[j], a = S.box_a[j];
+        const float2 b = S.box_b[j];
+        const float width = fmaxf(__fsub_rn(a.w, a.x), fmaxf(__fsub_rn(b.x, a.y), __fsub_rn(b.y, a.z)));
+        float4* t4 = reinterpret_cast<float4*>(tr + node);
+        t4[0] = c;
+        reinterpret_cast<int4*>(t4)[1] = make_int4(__float_as_int(width), k.x, k.y, k.z);
+        float4* b4 = reinterpret_cast<float4*>(bd + node);
+        b4[0] = a;
+        reinterpret_cast<int4*>(b4)[1] = make_int4(__float_as_int(b.x), __float_as_int(b.y), 0, k.w);
+        write_walk_node(wnp, node, make_float3(c.x, c.y, c.z), c.w, width, k.x, k.y, g, k.z,
+                            L.nseg > 1 ? (int)__ldg(L.seg_off + s) : 0, seg_end(s) - 1, ni);
+    }
+    __syncthreads();
+
+    if (threadIdx.x == 0) n_roots[blockIdx.x] = (uint32_t)S.n_roots;
+}
+
+// Climbs on from the subtrees the blocks' climbs left (one warp for each
+// run of kAggRange particles, one lane for each of its subtrees): a left child
+// hands its values to the relay and stops, a right child waits for the left
+// one's, computes the node and goes on.  The left child's particles, and so
+// its climber, come first, and blocks take their runs in launch order from a
+// ticket: whoever is waited for is running or done.  The wait is bounded.
+// A node above the blocks: its links, and which of it and its children are
+// FP64 nodes.
+struct RiseNode {
+    int node, cl, cr, re, up;  // node < 0: none
+    bool big, big_l, big_r;
+};
+__device__ __forceinline__ RiseNode rise_node(const BvhNodeTraverse* __restrict__ tr,
+                                              const BvhNodeBuild* __restrict__ bd, int node, int s, int ni, bool fp64) {
+    RiseNode r;
+    r.node = node < ni ? node : -1;
+    r.cl = r.cr = r.up = -1;
+    r.re = 0;
+    r.big = r.big_l = r.big_r = false;
+    if (r.node < 0) return r;
+    r.cl = __ldg(&tr[node].child_left);
+    r.cr = __ldg(&tr[node].child_right);
+    r.re = __ldg(&tr[node].range_end);
+    r.up = __ldg(&bd[node].parent);
+    // particles of the node and of its two children (the split is the left
+    // child's end of the range)
+    const int own = node + s, lo = min(own, r.re), hi = max(own, r.re);
+    const int split = r.cl >= ni ? r.cl - ni : r.cl + s;
+    r.big = fp64 && hi - lo + 1 >= kComFp64Min;
+    r.big_l = r.big && split - lo + 1 >= kComFp64Min;
+    r.big_r = r.big && hi - split >= kComFp64Min;
+    return r;
+}
+__device__ __forceinline__ bool valid_links(const RiseNode& n, int from, int lim) {
+    return n.cl >= 0 && n.cr >= 0 && n.cl < lim && n.cr < lim && (n.cl == from || n.cr == from);
+}
+struct RelayWords {
+    uint4 w0, w1;
+    uint2 w2;
+    ulonglong2 q0, q1;
+};
+__device__ __forceinline__ void relay_load(const WalkNode* wn, const BvhNodeTraverse* tr, const double4* com64,
+                                           const RiseNode& n, RelayWords& r) {
+    const uint4* w = reinterpret_cast<const uint4*>(wn + n.node);
+    r.w0 = load_relaxed(w);
+    r.w1 = load_relaxed(w + 1);
+    r.w2 = load_relaxed2(tr + n.node);
+    r.q0 = r.q1 = make_ulonglong2(0ull, 0ull);
+    if (n.big_l) {
+        r.q0 = load_relaxed64(com64 + n.node);
+        r.q1 = load_relaxed64(reinterpret_cast<const ulonglong2*>(com64 + n.node) + 1);
+    }
+}
+__device__ __forceinline__ bool relay_there(const RelayWords& r) {
+    return r.w0.x != ~0u && r.w0.y != ~0u && r.w0.z != ~0u && r.w0.w != ~0u && r.w1.x != ~0u && r.w1.y != ~0u &&
+           r.w1.z != ~0u && r.w1.w != ~0u && r.w2.x != ~0u && r.w2.y != ~0u && r.q0.x != ~0ull && r.q0.y != ~0ull &&
+           r.q1.x != ~0ull && r.q1.y != ~0ull;
+}
+__device__ __forceinline__ ChildData relay_values(const RelayWords& r) {
+    ChildData A;
+    A.lo = make_float3(__uint_as_float(r.w0.x), __uint_as_float(r.w0.y), __uint_as_float(r.w0.z));
+    A.hi = make_float3(__uint_as_float(r.w0.w), __uint_as_float(r.w1.x), __uint_as_float(r.w1.y));
+    A.com = make_float3(__uint_as_float(r.w1.z), __uint_as_float(r.w1.w), __uint_as_float(r.w2.x));
+    A.m = __uint_as_float(r.w2.y);
+    A.mx = make_double3(__longlong_as_double((long long)r.q0.x), __longlong_as_double((long long)r.q0.y),
+                        __longlong_as_double((long long)r.q1.x));
+    A.md = __longlong_as_double((long long)r.q1.y);
+    return A;
+}
+// The values of node n's left child, to its right child's climber.
+__device__ __forceinline__ void hand_over(WalkNode* wn, BvhNodeTraverse* tr, double4* com64, const RiseNode& n,
+                                          const ChildData& c) {
+    uint4* w = reinterpret_cast<uint4*>(wn + n.node);
+    store_relaxed(w, make_uint4(relay_word(c.lo.x), relay_word(c.lo.y), relay_word(c.lo.z), relay_word(c.hi.x)));
+    store_relaxed(w + 1, make_uint4(relay_word(c.hi.y), relay_word(c.hi.z), relay_word(c.com.x),
+                                    relay_word(c.com.y)));
+    store_relaxed(reinterpret_cast<uint2*>(tr + n.node), make_uint2(relay_word(c.com.z), relay_word(c.m)));
+    if (n.big_l) {
+        ulonglong2* q = reinterpret_cast<ulonglong2*>(com64 + n.node);
+        store_relaxed(q, make_ulonglong2(relay_word(c.mx.x), relay_word(c.mx.y)));
+        store_relaxed(q + 1, make_ulonglong2(relay_word(c.mx.z), relay_word(c.md)));
+    }
+}
+
+constexpr int kRiseWarps = 2;
+
+__global__ void __launch_bounds__(kRiseWarps * 32)
+rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restrict__ tr, BvhNodeBuild* __restrict__ bd,
+            double4* __restrict__ com64, const int32_t* __restrict__ leaf_parent, const int2* __restrict__ roots,
+            const uint32_t* __restrict__ n_roots, int n_runs, int com_fp64, WalkNodeParams wnp,
+            uint32_t* __restrict__ ticket, uint32_t* __restrict__ status) {
+    __shared__ int s_block;
+    if (threadIdx.x == 0) s_block = (int)atomicAdd(ticket, 1u);
+    __syncthreads();
+    const int run = s_block * kRiseWarps + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (run >= n_runs) return;
+    const int ni = L.n_internal;
+    const int lim = ni + L.n;
+    const int count = min((int)__ldg(n_roots + run), kAggRange);
+    const bool fp64 = com_fp64 != 0;
+    for (int r = lane; r < count; r += 32) {
+        // the finished subtree `from`, its values, and its parent
+        const int2 root = roots[run * kAggRange + r];
+        int from = root.x;
+        const int s = root.y;
+        ChildData mine;
+        int node;
+        if (from >= ni) {
+            const float4 p = __ldg(pos + (from - ni));
+            mine.lo = mine.hi = mine.com = make_float3(p.x, p.y, p.z);
+            mine.m = p.w;
+            node = __ldg(leaf_parent + (from - ni));
+        } else {
+            const float4 c = *reinterpret_cast<const float4*>(tr + from);
+            const float4 b_0 = *reinterpret_cast<const float4*>(bd + from);
+            const float4 b_1 = *(reinterpret_cast<const float4*>(bd + from) + 1);
+            mine.com = make_float3(c.x, c.y, c.z);
+            mine.m = c.w;
+            mine.lo = make_float3(b_0.x, b_0.y, b_0.z);
+            mine.hi = make_float3(b_0.w, b_1.x, b_1.y);
+            node = __float_as_int(b_1.w);
+        }
+        mine.mx = make_double3(0.0, 0.0, 0.0);
+        mine.md = 0.0;
+        const int seg_lo = L.nseg > 1 ? (int)__ldg(L.seg_off + s) : 0;
+        const int seg_hi = (L.nseg > 1 ? (int)__ldg(L.seg_off + s + 1) : L.n) - 1;
+        RiseNode N = rise_node(tr, bd, node, s, ni, fp64);
+        bool ok = N.node >= 0 && valid_links(N, from, lim);
+        if (ok && N.cl == from) {
+            hand_over(wnp.wn, tr, com64, N, mine);
+            continue;
+        }
+        RelayWords w;
+        if (ok) relay_load(wnp.wn, tr, com64, N, w);
+        RiseNode up = rise_node(tr, bd, ok ? N.up : -1, s, ni, fp64);
+        uint32_t polls = 0;
+        int levels = 0;
+        // a waiting lane polls once a turn, one that has its left child's
+        // values moves up one level
+        while (ok) {
+            if (!relay_there(w)) {
+                ok = ++polls < kRelayPolls;
+                relay_load(wnp.wn, tr, com64, N, w);
+                continue;
+            }
+            const ChildData A = relay_values(w);
+            ChildData next;
+            const float width = merge_children(A, mine, next);
+            next.md = 0.0;
+            next.mx = make_double3(0.0, 0.0, 0.0);
+            const bool sums = N.big && next.m > 0.0f;
+            if (sums) {
                 double3 amx, bmx;
                 double amd, bmd;
-                fp64_terms(A, big_l, amx, amd);
-                fp64_terms(B, big_r, bmx, bmd);
+                fp64_terms(A, N.big_l, amx, amd);
+                fp64_terms(mine, N.big_r, bmx, bmd);
                 next.md = amd + bmd;
                 next.mx = make_double3(amx.x + bmx.x, amx.y + bmx.y, amx.z + bmx.z);
-                com = make_float3((float)(next.mx.x / next.md), (float)(next.mx.y / next.md),
-                                  (float)(next.mx.z / next.md));
+                next.com = make_float3(0.0f, 0.0f, 0.0f);  // below: a parent takes the sums instead
             } else {
-                com = make_float3(com_fp32(A.com.x, A.m, B.com.x, B.m, m), com_fp32(A.com.y, A.m, B.com.y, B.m, m),
-                                  com_fp32(A.com.z, A.m, B.com.z, B.m, m));
+                next.com = merged_com_fp32(A, mine, next);
             }
-        } else {
-            com = make_float3(__fmul_rn(__fadd_rn(lo.x, hi.x), 0.5f), __fmul_rn(__fadd_rn(lo.y, hi.y), 0.5f),
-                              __fmul_rn(__fadd_rn(lo.z, hi.z), 0.5f));
+            // the parent first: its other child may be waiting, and its words
+            // and links travel while this node's record is finished
+            const RiseNode cur = N;
+            const bool more = up.node >= 0 && cur.up >= 0;
+            ok = !more ? cur.up < 0 : valid_links(up, cur.node, lim) && ++levels <= kAggMaxLevels;
+            const bool hand = ok && more && up.cl == cur.node;
+            if (sums && ok && more && !(hand ? up.big_l : up.big_r)) ok = false;  // FP64 nodes have FP64 parents
+            if (hand && ok) hand_over(wnp.wn, tr, com64, up, next);
+            N = up;
+            if (ok && more && !hand) {
+                relay_load(wnp.wn, tr, com64, N, w);
+                up = rise_node(tr, bd, N.up, s, ni, fp64);
+            }
+            if (sums)
+                next.com = make_float3((float)(next.mx.x / next.md), (float)(next.mx.y / next.md),
+                                       (float)(next.mx.z / next.md));
+            com64[cur.node] = make_double4(next.mx.x, next.mx.y, next.mx.z, next.md);
+            reinterpret_cast<float4*>(tr + cur.node)[0] = make_float4(next.com.x, next.com.y, next.com.z, next.m);
+            tr[cur.node].width = width;
+            float4* b4 = reinterpret_cast<float4*>(bd + cur.node);
+            b4[0] = make_float4(next.lo.x, next.lo.y, next.lo.z, next.hi.x);
+            reinterpret_cast<float2*>(b4 + 1)[0] = make_float2(next.hi.y, next.hi.z);
+            write_walk_node(wnp, cur.node, next.com, next.m, width, cur.cl, cur.cr, cur.node + s, cur.re, seg_lo,
+                            seg_hi, ni);
+            if (!ok || !more || hand) break;
+            mine = next;
+            polls = 0;
         }
-        if (big) com64[node] = make_double4(next.mx.x, next.mx.y, next.mx.z, next.md);
-        float4* t4 = reinterpret_cast<float4*>(tr + node);
-        t4[0] = make_float4(com.x, com.y, com.z, m);
-        tr[node].width = width;
-        if (wnp.wn) write_walk_node(wnp, node, com, m, width, cl, cr, own, re, seg_lo, seg_hi, ni);
-        float4* b4 = reinterpret_cast<float4*>(bd + node);
-        b4[0] = make_float4(lo.x, lo.y, lo.z, hi.x);
-        reinterpret_cast<float2*>(b4 + 1)[0] = make_float2(hi.y, hi.z);
-        next.lo = lo;
-        next.hi = hi;
-        next.com = com;
-        next.m = m;
-        if (local) {
-            LocalNode& q = snode[own - b0];
-            q.lo = lo;
-            q.hi = hi;
-            q.com = com;
-            q.m = m;
-        }
-        mine = next;
-        from = node;
-        node = up;
-        cl = ncl;
-        cr = ncr;
-        up = nup;
-        re = nre;
-        have = node >= 0;  // the root ends the climb
+        if (!ok) atomicOr(status, GCS_DEV_TREE_MALFORMED);
     }
+}
+
+// Empty relay words of every node above the blocks, and the block ticket, for
+// an aggregation that does not follow a build (one thread per particle, as in
+// walk_nodes_kernel).
+__global__ void relay_reset_kernel(Layout L, BvhNodeTraverse* __restrict__ tr, WalkNode* __restrict__ wn,
+                                   double4* __restrict__ com64, uint32_t* __restrict__ ticket) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g == 0) *ticket = 0u;
+    if (g >= L.n) return;
+    const int s = L.nseg > 1 ? __ldg(L.seg_id + g) : 0;
+    if (g + 1 >= (int)__ldg(L.seg_off + s + 1)) return;
+    const int re = tr[g - s].range_end;
+    if (above_blocks(min(g, re), max(g, re))) relay_clear(wn, tr, com64, g - s);
 }
 
 int tree_grid(int64_t n) {
@@ -428,18 +622,27 @@ int tree_grid(int64_t n) {
 }  // namespace
 
 void launch_build(const Layout& L, const uint64_t* keys, BvhNodeTraverse* tr, BvhNodeBuild* bd,
-                  int32_t* leaf_parent, uint32_t* status, cudaStream_t st) {
+                  int32_t* leaf_parent, WalkNode* wn, double4* com64, uint32_t* agg_ticket, uint32_t* status,
+                  cudaStream_t st) {
     if (L.n <= 0) return;
-    build_kernel<<<tree_grid(L.n), 256, 0, st>>>(L, keys, tr, bd, leaf_parent, status);
+    build_kernel<<<tree_grid(L.n), 256, 0, st>>>(L, keys, tr, bd, leaf_parent, wn, com64, agg_ticket, status);
+}
+
+void launch_relay_reset(const Layout& L, BvhNodeTraverse* tr, WalkNode* wn, double4* com64, uint32_t* agg_ticket,
+                        cudaStream_t st) {
+    if (L.n <= 0) return;
+    relay_reset_kernel<<<tree_grid(L.n), 256, 0, st>>>(L, tr, wn, com64, agg_ticket);
 }
 
 void launch_aggregate(const Layout& L, const float4* pos, BvhNodeTraverse* tr, BvhNodeBuild* bd,
                       double4* com64, const int32_t* leaf_parent, int com_fp64, const WalkNodeParams& wnp,
-                      uint32_t* status, cudaStream_t st) {
+                      int2* roots, uint32_t* n_roots, uint32_t* agg_ticket, uint32_t* status, cudaStream_t st) {
     if (L.n <= 0) return;
-    const unsigned blocks = (unsigned)((L.n + kAggRange - 1) / kAggRange);
-    aggregate_kernel<<<blocks, kAggThreads, 0, st>>>(L, pos, tr, bd, com64, leaf_parent, com_fp64,
-                                                             wnp, status);
+    const int runs = (L.n + kAggRange - 1) / kAggRange;
+    aggregate_kernel<<<(unsigned)runs, kAggThreads, 0, st>>>(L, pos, tr, bd, leaf_parent, wnp, roots, n_roots, status);
+    if (runs > 1)  // one block's nodes are all local
+        rise_kernel<<<(unsigned)((runs + kRiseWarps - 1) / kRiseWarps), kRiseWarps * 32, 0, st>>>(
+            L, pos, tr, bd, com64, leaf_parent, roots, n_roots, runs, com_fp64, wnp, agg_ticket, status);
 }
 
 void launch_walk_nodes(const Layout& L, const BvhNodeTraverse* tr, WalkNodeParams wnp, uint32_t* status,
