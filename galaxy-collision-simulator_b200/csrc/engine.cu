@@ -96,6 +96,8 @@ struct gcs_ctx {
     int64_t* targets = nullptr;
     int64_t targets_cap = 0;
     double* direct_out = nullptr;
+    double* direct_sums = nullptr;  // work space of the direct sum's source splits
+    size_t direct_sums_cap = 0;
     unsigned long long* counts = nullptr;  // walk interaction counters (count mode)
     int2* walk_stack = nullptr;            // per-warp global bottoms of the walk stacks
     // splat renderer: fixed-point accumulator and RGBA staging, sized for
@@ -287,7 +289,7 @@ void free_all(gcs_ctx* c) {
                     c->idx[0], c->idx[1], c->tr, c->bd, c->wn, c->com64, c->leaf_parent, c->seg_off,
                     c->seg_id, c->groups, c->supers, c->sg_list, c->sg_src, c->sg_meta, c->perm, c->split_sums, c->split_arrived, c->chunks,
                     c->seg_bounds, c->staging, c->pb_staging,
-                    c->scratch, c->status, c->diag, c->targets, c->direct_out, c->counts,
+                    c->scratch, c->status, c->diag, c->targets, c->direct_out, c->direct_sums, c->counts,
                     c->walk_stack, c->render_acc, c->render_rgba, c->star_chunk_done};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -1619,10 +1621,19 @@ int gcs_direct_accels_fp64(gcs_ctx* c, const gcs_params* p, int32_t segment,
             return GCS_ERR_NOMEM;
         c->targets_cap = n_targets;
     }
+    const int splits = direct_splits(n, n_targets);
+    const size_t sums = splits > 1 ? 3 * (size_t)n_targets * (size_t)splits : 0;
+    if (sums > c->direct_sums_cap) {
+        if (c->direct_sums) cudaFree(c->direct_sums);
+        c->direct_sums = nullptr;
+        c->direct_sums_cap = 0;
+        if (dalloc(c, &c->direct_sums, sums)) return GCS_ERR_NOMEM;
+        c->direct_sums_cap = sums;
+    }
     GCS_CUDA(c, cudaMemcpyAsync(c->targets, targets, sizeof(int64_t) * (size_t)n_targets,
                                 cudaMemcpyHostToDevice, c->stream));
-    launch_direct_fp64(c->pos[c->cur], first, n, c->targets, n_targets, (double)p->G,
-                       (double)p->epsilon_sq, c->direct_out, c->stream);
+    launch_direct_fp64(c->pos[c->cur], first, n, c->targets, n_targets, splits, (double)p->G,
+                       (double)p->epsilon_sq, c->direct_sums, c->direct_out, c->stream);
     int rc = check_launch(c, "direct_fp64");
     if (rc) return rc;
     GCS_CUDA(c, cudaMemcpyAsync(out, c->direct_out, sizeof(double) * 3 * (size_t)n_targets,

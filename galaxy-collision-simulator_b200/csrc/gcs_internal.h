@@ -313,7 +313,12 @@ void launch_splat_playback(const PlaybackStar* recs, int64_t n, const float* vie
                            int height, unsigned long long* acc, cudaStream_t st);
 void launch_resolve(const unsigned long long* acc, int64_t pixels, uint8_t* rgba, cudaStream_t st);
 
+// FP64 direct sums of n_targets particles; sums: 3 * n_targets * splits
+// doubles of work space when splits > 1.
+constexpr int64_t kDirectMaxSplits = 1024;
+int direct_splits(int64_t seg_n, int64_t n_targets);
 void launch_direct_fp64(const float4* pos, int64_t seg_first, int64_t seg_n, const int64_t* targets,
-                        int64_t n_targets, double G, double eps2, double* out, cudaStream_t st);
+                        int64_t n_targets, int splits, double G, double eps2, double* sums, double* out,
+                        cudaStream_t st);
 
 }  // namespace gcs

@@ -115,3 +115,31 @@ def test_precision_runner_small(gcs_mod, capsys):
         assert [c["step"] for c in r["checkpoints"]] == [0, 10, 20]
         assert 0 < r["median_force_error"] < 1e-2
         assert r["max_abs_dE_rel"] < 1e-2
+
+
+@pytest.mark.parametrize("eps2", [0.0, 1e-4])
+@pytest.mark.parametrize("n_targets", [1, 3, 4, 5, 37])
+@pytest.mark.parametrize("n", [1, 2, 700, 5000])
+def test_direct_fp64_any_targets(gcs_mod, n, n_targets, eps2):
+    """Targets in any order and repeated, target tiles that are not full, one
+    and several source splits (1,024 sources each), no softening; segment 1 of
+    two.  Bound: (n + 16) roundings of the terms' absolute sum, 8 per term."""
+    gcs = gcs_mod
+    rng = np.random.default_rng(n + n_targets)
+    stars = np.zeros(n + 9, gcs.STAR_DTYPE)
+    for f in ("x", "y", "z"):
+        stars[f] = rng.normal(0, 3, n + 9).astype(np.float32)
+    stars["mass"] = rng.random(n + 9).astype(np.float32)
+    tg = rng.integers(0, n, n_targets)
+    p = gcs.reference_params(epsilon_sq=eps2, G=1.5)
+    with gcs.Context(n + 9, 2) as ctx:
+        ctx.set_segments([9, n])
+        ctx.upload(stars)
+        got = ctx.direct_fp64(p, tg, segment=1)
+    x = np.stack([stars[f][9:] for f in ("x", "y", "z")], 1).astype(np.float64)
+    m = stars["mass"][9:].astype(np.float64)
+    for k, t in enumerate(tg):
+        d = np.delete(x - x[t], t, 0)
+        r2 = (d * d).sum(1) + float(p.epsilon_sq)
+        term = p.G * (np.delete(m, t) / (r2 * np.sqrt(r2)))[:, None] * d
+        assert np.all(np.abs(got[k] - term.sum(0)) <= 8 * (n + 16) * 2.0 ** -53 * np.abs(term).sum(0))
