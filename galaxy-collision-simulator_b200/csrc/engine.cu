@@ -20,6 +20,7 @@
 #include <cuda.h>  // driver API types for the pointer-range query (entry point fetched at run time)
 
 #include "gcs_internal.h"
+#include "host_copy.h"
 
 using namespace gcs;
 
@@ -123,6 +124,7 @@ struct gcs_ctx {
     uint32_t* star_flags_dev = nullptr;  // its device address
     uint32_t* star_chunk_done = nullptr;
     uint32_t star_epoch = 0;
+    HostCopy* host_copy = nullptr;       // copies into pageable memory (taken at the first one)
     size_t walk_stack_entries = 0;
     int32_t group_width = 32;              // targets per walk group (<= 64; two per lane above 32)
     bool walk_frontier = true;             // super-group frontier pass before the walk
@@ -285,6 +287,7 @@ void free_all(gcs_ctx* c) {
     if (c->gather_fork) cudaEventDestroy(c->gather_fork);
     if (c->gather_join) cudaEventDestroy(c->gather_join);
     if (c->star_flags) cudaFreeHost(c->star_flags);
+    if (c->host_copy) HostCopy::release();
     void* ptrs[] = {c->pos[0], c->pos[1], c->vel[0], c->vel[1], c->acc, c->keys[0], c->keys[1],
                     c->idx[0], c->idx[1], c->tr, c->bd, c->wn, c->com64, c->leaf_parent, c->seg_off,
                     c->seg_id, c->groups, c->supers, c->sg_list, c->sg_src, c->sg_meta, c->perm, c->split_sums, c->split_arrived, c->chunks,
@@ -455,6 +458,27 @@ int upload_groups(gcs_ctx* c) {
 }
 
 }  // namespace
+
+// The process's pageable-copy threads, taken for one copy of `bytes` into
+// host; nullptr: copy plainly (pinned or small, or another thread has them).
+static HostCopy* begin_host_copy(gcs_ctx* c, const void* host, size_t bytes) {
+    if (bytes < HostCopy::kWorth || !is_pageable(host)) return nullptr;
+    if (!c->host_copy) c->host_copy = HostCopy::acquire();
+    return c->host_copy && c->host_copy->begin() ? c->host_copy : nullptr;
+}
+
+// Copy device memory to the caller's host memory on the context stream; the
+// stream is idle when it returns.
+static int copy_to_host(gcs_ctx* c, void* host, const void* src, size_t bytes) {
+    if (HostCopy* hc = begin_host_copy(c, host, bytes)) {
+        hc->add(host, src, bytes, c->stream);
+        GCS_CUDA(c, hc->finish());
+    } else {
+        GCS_CUDA(c, cudaMemcpyAsync(host, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+    }
+    GCS_CUDA(c, cudaStreamSynchronize(c->stream));
+    return GCS_OK;
+}
 
 // The partition's second stream and its fork/join events, created once per
 // context (before any capture of the step: build_step_graphs calls it too).
@@ -1014,10 +1038,7 @@ int gcs_download_stars(gcs_ctx* c, Star* host, int64_t offset, int64_t n) {
                       c->stream);
     int rc = check_launch(c, "pack");
     if (rc) return rc;
-    GCS_CUDA(c, cudaMemcpyAsync(host, c->staging + offset, sizeof(Star) * (size_t)n,
-                                cudaMemcpyDeviceToHost, c->stream));
-    GCS_CUDA(c, cudaStreamSynchronize(c->stream));
-    return GCS_OK;
+    return copy_to_host(c, host, c->staging + offset, sizeof(Star) * (size_t)n);
 }
 
 int gcs_download_playback(gcs_ctx* c, PlaybackStar* host, int64_t offset, int64_t n) {
@@ -1028,10 +1049,7 @@ int gcs_download_playback(gcs_ctx* c, PlaybackStar* host, int64_t offset, int64_
                          n, c->stream);
     int rc = check_launch(c, "pack_playback");
     if (rc) return rc;
-    GCS_CUDA(c, cudaMemcpyAsync(host, c->pb_staging + offset, sizeof(PlaybackStar) * (size_t)n,
-                                cudaMemcpyDeviceToHost, c->stream));
-    GCS_CUDA(c, cudaStreamSynchronize(c->stream));
-    return GCS_OK;
+    return copy_to_host(c, host, c->pb_staging + offset, sizeof(PlaybackStar) * (size_t)n);
 }
 
 // Capture the full step twice, once from each ping-pong parity of the
@@ -1253,10 +1271,12 @@ static int step_host_overlapped(gcs_ctx* c, const gcs_params* p, Star* host, int
     const int ng = c->n_groups;
     const int64_t resident = walk_grid_blocks(ng, p->walk_blocks_per_sm, c->sm_count, p->with_potential) *
                              (int64_t)kWalkBlockWarps;
+    // (chunks of at least a piece of the threaded copy)
+    const int least = (int)(HostCopy::kPiece / sizeof(Star) * (size_t)ng / (size_t)c->n) + 1;
     const int tail_groups = (int)std::min<int64_t>(ng, 2 * resident);
     const int head_groups = ng - tail_groups;
-    const int hpc = head_groups > 0 ? (head_groups + kMaxStarHeadChunks - 1) / kMaxStarHeadChunks : 1;
-    const int tpc = (tail_groups + kMaxStarTailChunks - 1) / kMaxStarTailChunks;
+    const int hpc = std::max(least, head_groups > 0 ? (head_groups + kMaxStarHeadChunks - 1) / kMaxStarHeadChunks : 1);
+    const int tpc = std::max(least, (tail_groups + kMaxStarTailChunks - 1) / kMaxStarTailChunks);
     // chunk boundaries (group indices): large chunks over the head, small
     // ones over the tail; with partitioned super-groups each boundary moves
     // up to the next super-group edge, so a chunk's particles stay one range
@@ -1300,12 +1320,14 @@ static int step_host_overlapped(gcs_ctx* c, const gcs_params* p, Star* host, int
     // Copy each chunk once its flag is up; when the walk has finished, copy
     // what is left (a chunk that was never signalled is reported).
     bool missing = false;
+    HostCopy* hc = nullptr;  // begun with the first chunk
     for (int k = 0; k < chunks && !rc; ++k) {
         const int g0 = bound[(size_t)k], g1 = bound[(size_t)k + 1];
         const int64_t first = c->h_group_start[(size_t)g0];
         const int64_t end = g1 < ng ? c->h_group_start[(size_t)g1] : c->n;
         for (uint32_t polls = 1;; ++polls) {
             if (__atomic_load_n(c->star_flags + k, __ATOMIC_ACQUIRE) == epoch) break;
+            if (hc && (polls & 7u) == 0u) hc->work();  // pieces that have landed
             if ((polls & 63u) == 0u) {
                 const cudaError_t q = cudaEventQuery(c->star_walked);
                 if (q == cudaSuccess) {
@@ -1320,6 +1342,11 @@ static int step_host_overlapped(gcs_ctx* c, const gcs_params* p, Star* host, int
             }
         }
         if (rc) break;
+        if (k == 0) hc = begin_host_copy(c, host, sizeof(Star) * (size_t)c->n);
+        if (hc) {
+            hc->add(host + first, c->staging + first, sizeof(Star) * (size_t)(end - first), c->star_stream);
+            continue;
+        }
         const cudaError_t e = cudaMemcpyAsync(host + first, c->staging + first, sizeof(Star) * (size_t)(end - first),
                                               cudaMemcpyDeviceToHost, c->star_stream);
         if (e != cudaSuccess) {
@@ -1328,11 +1355,12 @@ static int step_host_overlapped(gcs_ctx* c, const gcs_params* p, Star* host, int
         }
     }
     // no copy into the caller's buffer may outlive this call
+    const cudaError_t e0 = hc ? hc->finish() : cudaSuccess;
     const cudaError_t e1 = cudaStreamSynchronize(c->star_stream);
     const cudaError_t e2 = cudaStreamSynchronize(c->stream);
     if (rc) return rc;
-    if (e1 != cudaSuccess || e2 != cudaSuccess) {
-        set_error(c, "cudaStreamSynchronize (host step)", e1 != cudaSuccess ? e1 : e2);
+    if (e0 != cudaSuccess || e1 != cudaSuccess || e2 != cudaSuccess) {
+        set_error(c, "host step copies", e0 != cudaSuccess ? e0 : e1 != cudaSuccess ? e1 : e2);
         return GCS_ERR_CUDA;
     }
     if (missing) {
@@ -1748,11 +1776,7 @@ int gcs_render_frame(gcs_ctx* c, const gcs_camera* cam, int32_t segment, int32_t
     launch_resolve(c->render_acc, pixels, target, c->stream);
     int rc = check_launch(c, "render");
     if (rc) return rc;
-    if (rgba_on_host) {
-        GCS_CUDA(c, cudaMemcpyAsync(rgba, c->render_rgba, 4 * (size_t)pixels, cudaMemcpyDeviceToHost, c->stream));
-        GCS_CUDA(c, cudaStreamSynchronize(c->stream));
-    }
-    return GCS_OK;
+    return rgba_on_host ? copy_to_host(c, rgba, c->render_rgba, 4 * (size_t)pixels) : GCS_OK;
 }
 
 int gcs_render_stars(const Star* stars, int64_t n, const gcs_camera* cam, int32_t width, int32_t height,

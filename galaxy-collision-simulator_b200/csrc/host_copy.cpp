@@ -1,0 +1,231 @@
+// host_copy.cpp - see host_copy.h.
+#include "host_copy.h"
+
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <cstdint>
+#include <cstring>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace gcs {
+
+namespace {
+
+inline void relax() {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+}
+
+std::mutex g_mu;
+HostCopy* g_copy = nullptr;
+int g_users = 0;
+
+}  // namespace
+
+struct HostCopy::Impl {
+    struct Piece {
+        char* dst;
+        size_t bytes;
+    };
+    char* ring = nullptr;                 // pinned, kSlots pieces
+    cudaEvent_t landed_ev[kSlots] = {};   // of the device current at begin()
+    int device = -1;
+    Piece piece[kSlots];
+    // piece numbers, never reset
+    std::atomic<uint64_t> landed{0};      // pieces whose device copy is done
+    std::atomic<uint64_t> claimed{0};     // pieces taken by a copying thread
+    std::atomic<uint64_t> done[kSlots];   // piece number + 1 last copied out of the slot
+    uint64_t queued = 0;                  // owner's
+    cudaError_t error = cudaSuccess;      // owner's
+    std::mutex own;                       // the running copy
+    std::mutex mu;                        // wakes the helpers
+    std::condition_variable cv;
+    std::atomic<bool> active{false};
+    bool stop = false;
+    std::vector<std::thread> threads;
+
+    bool copy_one() {
+        uint64_t i = claimed.load(std::memory_order_relaxed);
+        if (i >= landed.load(std::memory_order_acquire)) return false;
+        if (!claimed.compare_exchange_strong(i, i + 1, std::memory_order_relaxed)) return false;
+        const int s = (int)(i % kSlots);
+        std::memcpy(piece[s].dst, ring + (size_t)s * kPiece, piece[s].bytes);
+        done[s].store(i + 1, std::memory_order_release);
+        return true;
+    }
+    void help() {
+        for (;;) {
+            {
+                std::unique_lock<std::mutex> lk(mu);
+                cv.wait(lk, [&] { return stop || active.load(std::memory_order_relaxed); });
+                if (stop) return;
+            }
+            while (active.load(std::memory_order_relaxed))
+                if (!copy_one()) relax();
+        }
+    }
+    void drop_events() {
+        for (cudaEvent_t& e : landed_ev) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+        device = -1;
+    }
+    ~Impl() {
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            stop = true;
+        }
+        cv.notify_all();
+        for (std::thread& t : threads) t.join();
+        drop_events();
+        if (ring) cudaFreeHost(ring);
+    }
+};
+
+HostCopy::~HostCopy() { delete impl; }
+
+HostCopy* HostCopy::acquire() {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (!g_copy) {
+        const int cores = (int)std::thread::hardware_concurrency();
+        if (cores < 2) return nullptr;
+        Impl* im = new Impl();
+        for (auto& d : im->done) d.store(0, std::memory_order_relaxed);
+        if (cudaHostAlloc(reinterpret_cast<void**>(&im->ring), kPiece * kSlots, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            im->ring = nullptr;
+            delete im;
+            return nullptr;
+        }
+        try {
+            for (int k = 0; k < std::min(kWorkers, cores - 1); ++k) im->threads.emplace_back([im] { im->help(); });
+        } catch (...) {  // fewer threads, or none: the caller's own still copies
+        }
+        g_copy = new HostCopy();
+        g_copy->impl = im;
+    }
+    ++g_users;
+    return g_copy;
+}
+
+void HostCopy::release() {
+    HostCopy* last = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (--g_users == 0) {
+            last = g_copy;
+            g_copy = nullptr;
+        }
+    }
+    delete last;
+}
+
+bool HostCopy::begin() {
+    Impl& m = *impl;
+    if (!m.own.try_lock()) return false;
+    int dev = -1;
+    bool ok = cudaGetDevice(&dev) == cudaSuccess;
+    if (ok && dev != m.device) {  // events belong to a device
+        m.drop_events();
+        for (cudaEvent_t& e : m.landed_ev)
+            ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+        if (ok) m.device = dev;
+        else m.drop_events();
+    }
+    if (!ok) {
+        cudaGetLastError();
+        m.own.unlock();
+        return false;
+    }
+    // the counters go on from the last copy (a helper may still be looking at
+    // them); pieces that an error kept from landing are numbered again
+    m.queued = m.landed.load(std::memory_order_relaxed);
+    m.error = cudaSuccess;
+    {
+        std::lock_guard<std::mutex> lk(m.mu);
+        m.active.store(true, std::memory_order_release);
+    }
+    m.cv.notify_all();
+    return true;
+}
+
+// Take note of pieces that have landed (in order).
+void HostCopy::poll() {
+    Impl& m = *impl;
+    uint64_t i = m.landed.load(std::memory_order_relaxed);
+    while (i < m.queued && m.error == cudaSuccess) {
+        const cudaError_t e = cudaEventQuery(m.landed_ev[i % kSlots]);
+        if (e == cudaErrorNotReady) break;
+        if (e != cudaSuccess) {
+            m.error = e;
+            break;
+        }
+        m.landed.store(++i, std::memory_order_release);
+    }
+}
+
+void HostCopy::work() {
+    poll();
+    if (!impl->copy_one()) relax();
+}
+
+void HostCopy::add(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    Impl& m = *impl;
+    for (size_t at = 0; at < bytes && m.error == cudaSuccess; at += kPiece) {
+        const uint64_t i = m.queued;
+        const int s = (int)(i % kSlots);
+        // the slot's last piece has been copied out
+        while (i >= kSlots && m.done[s].load(std::memory_order_acquire) != i - kSlots + 1 && m.error == cudaSuccess)
+            work();
+        if (m.error != cudaSuccess) return;
+        m.piece[s].dst = static_cast<char*>(dst) + at;
+        m.piece[s].bytes = std::min(kPiece, bytes - at);
+        cudaError_t e = cudaMemcpyAsync(m.ring + (size_t)s * kPiece, static_cast<const char*>(src) + at,
+                                        m.piece[s].bytes, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaEventRecord(m.landed_ev[s], st);
+        if (e != cudaSuccess) {
+            m.error = e;
+            return;
+        }
+        m.queued = i + 1;
+        poll();
+    }
+}
+
+cudaError_t HostCopy::finish() {
+    Impl& m = *impl;
+    const auto copied = [&] {
+        const uint64_t n = m.landed.load(std::memory_order_relaxed);
+        // every landed piece: the last kSlots of them say so themselves, the
+        // ones before made room for them
+        for (uint64_t i = n > kSlots ? n - kSlots : 0; i < n; ++i)
+            if (m.done[i % kSlots].load(std::memory_order_acquire) != i + 1) return false;
+        return true;
+    };
+    while (m.error == cudaSuccess && m.landed.load(std::memory_order_relaxed) < m.queued) work();
+    while (!copied()) work();
+    // after an error no device copy may still be on its way into the ring
+    if (m.error != cudaSuccess)
+        for (int s = 0; s < kSlots; ++s)
+            if (m.landed_ev[s]) cudaEventSynchronize(m.landed_ev[s]);
+    m.active.store(false, std::memory_order_release);
+    const cudaError_t e = m.error;
+    m.own.unlock();
+    return e;
+}
+
+bool is_pageable(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+}  // namespace gcs

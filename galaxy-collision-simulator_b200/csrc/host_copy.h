@@ -1,0 +1,56 @@
+// host_copy.h - device-to-host copies into pageable memory, through pinned
+// pieces and several threads.
+//
+// A plain cudaMemcpyAsync into pageable memory is staged by the driver on the
+// calling thread: about 17 GB/s (9.6 MB: 573 us, 186 us when pinned), plus
+// some 15 us a call.  Here the device copies pieces of kPiece bytes into a
+// ring of pinned ones at PCIe speed, and the calling thread and up to
+// kWorkers helpers copy the pieces that have landed into the caller's memory
+// (also spreading the page faults of memory not touched before).  Measured
+// with 16 cores: 9.6 MB of Stars 638 -> 340 us, a host step of 300,000
+// particles into pageable memory 1,529 -> 651 us (its 64 plain chunk copies
+// cost more than its walk), a 1920 x 1080 frame 799 -> 557 us.  Two, four and
+// eight threads copy 9.6 MB in 358, 264 and 423 us.
+//
+// One ring and its threads serve the process: made by the first context that
+// uses them, kept while such a context lives, given back with the last.  A
+// copy takes them for itself (begin() fails while another thread has them,
+// and callers then copy plainly).
+#pragma once
+#include <cstddef>
+#include <cuda_runtime.h>
+
+namespace gcs {
+
+class HostCopy {
+  public:
+    static constexpr size_t kPiece = 512 << 10;
+    static constexpr int kSlots = 8;
+    static constexpr int kWorkers = 3;
+    static constexpr size_t kWorth = 1 << 20;  // smaller copies go plainly
+
+    // The process's instance, counted by user; nullptr where there is no
+    // pinned memory or no second core.
+    static HostCopy* acquire();
+    static void release();
+
+    bool begin();  // take it; false: busy
+    // Queue a copy of `bytes` from device memory on `st`; blocks (working on
+    // landed pieces) while the ring is full.  Nothing is queued after an error.
+    void add(void* dst, const void* src, size_t bytes, cudaStream_t st);
+    void work();            // copy one landed piece, if there is one
+    cudaError_t finish();   // wait for everything queued, and give it back
+
+  private:
+    struct Impl;
+    Impl* impl = nullptr;
+    HostCopy() = default;
+    ~HostCopy();
+    void poll();
+};
+
+// Whether p is ordinary pageable host memory (false: pinned, managed or
+// device memory, which cudaMemcpyAsync copies to directly).
+bool is_pageable(const void* p);
+
+}  // namespace gcs
