@@ -493,8 +493,8 @@ int gcs_render_playback(const PlaybackStar* frame, int64_t n, const gcs_camera* 
  * gcs_server_submit; every gcs_server_tick admits queued scenarios in
  * arrival order while segment slots and particle capacity allow, lays the
  * resident scenarios out as segments of one context (kept scenarios stay
- * on the device; the step graph is captured again only after a membership
- * change), advances all of them by one step with one launch per stage, and
+ * on the device; a membership that lasts 16 rounds steps as a captured graph
+ * from then on), advances all of them by one step with one launch per stage, and
  * retires those that reached their step count.  Each scenario's final
  * Stars are byte-identical to stepping it alone with the same parameters.
  * Not thread-safe: one host thread drives a server. */

@@ -160,3 +160,30 @@ def test_server_budget_and_capacity(gcs_mod):
             if len(ids) == 2:
                 break
         assert ids == [1, 2]
+
+
+def test_server_switches_to_graphs_and_back(gcs_mod):
+    """Memberships that last longer than the 16 plain rounds step as graphs
+    until the next change; results stay those of stepping alone."""
+    gcs = gcs_mod
+    p = _params(gcs)
+    a, b = (s for s, _ in _scenarios(gcs, 2, seed0=31))
+    with gcs.Server(p, len(a) + len(b), 2, 8e9) as srv:
+        builds = lambda: int(gcs.lib().gcs_graph_builds(gcs.lib().gcs_server_context(srv._h)))  # noqa: E731
+        srv.submit(0, a, 40)
+        for _ in range(16):
+            srv.tick()
+        assert builds() == 0
+        srv.tick()
+        assert builds() == 1
+        srv.submit(1, b, 23)  # a change: plain rounds again, then another capture
+        while srv.counts()[2] < 2:
+            srv.tick()
+        assert builds() == 2
+        got = {}
+        for _ in range(2):
+            info, stars = srv.pop()
+            got[int(info.id)] = stars
+    for sid, (st, steps) in enumerate(((a, 40), (b, 23))):
+        ref, _ = _solo(gcs, st, p, steps)
+        assert got[sid].tobytes() == ref.tobytes()
