@@ -48,6 +48,7 @@ struct gcs_ctx {
     uint64_t* keys[2] = {nullptr, nullptr};
     uint32_t* idx[2] = {nullptr, nullptr};
     int sorted_buf = 0;
+    bool front = false;  // small scenarios sort in one launch (k_front.cu)
     BvhNodeTraverse* tr = nullptr;
     BvhNodeBuild* bd = nullptr;
     // Walk records (one per internal node) and what they were written for:
@@ -666,7 +667,19 @@ static int run_stages(gcs_ctx* c, const gcs_params* p, int first, int last) {
     }
     const bool gather_beside_build = first <= GCS_STAGE_GATHER && last >= GCS_STAGE_BUILD;
     const bool kick_in_walk = first <= GCS_STAGE_WALK && last >= GCS_STAGE_INTEGRATE && c->range_count < 0;
-    for (int s = first; s <= last; ++s) {
+    int s = first;
+    if (first <= GCS_STAGE_ENCODE && last >= GCS_STAGE_SORT && c->nseg == 1 && c->n <= kFrontMax && c->front) {
+        // a small scenario: bounds, encode and sort in one launch
+        const int bounds = p->bounds_mode != GCS_BOUNDS_DEVICE ? kFrontBoundsCaller
+                         : first == GCS_STAGE_BOUNDS ? kFrontBoundsReduce : kFrontBoundsGiven;
+        c->sorted_buf = 0;  // as after kKeyPasses passes
+        launch_front(c->pos[c->cur], c->n, bounds, p->global_min, p->global_max, c->seg_bounds, c->keys[0], c->idx[0],
+                     c->status, c->stream);
+        rc = check_launch(c, "bounds, encode and sort");
+        if (rc) return rc;
+        s = GCS_STAGE_GATHER;
+    }
+    for (; s <= last; ++s) {
         rc = run_stage(c, p, s, gather_beside_build, kick_in_walk);
         if (rc) return rc;
     }
@@ -749,6 +762,7 @@ int gcs_create(gcs_ctx** out, int64_t capacity, int32_t max_segments, int32_t de
         delete c;
         return GCS_ERR_NOMEM;
     }
+    c->front = front_available();
     cudaMemset(c->scratch, 0, c->scratch_cap);  // the walk queue starts (and stays) at zero
     cudaMemset(c->status, 0, sizeof(uint32_t));
     cudaMemset(c->split_arrived, 0, sizeof(uint32_t) * split_units((size_t)capacity, max_segments));

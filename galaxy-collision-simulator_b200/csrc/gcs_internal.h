@@ -125,6 +125,23 @@ void launch_encode(const Layout& L, const float4* pos, int bounds_mode, float gm
                    const float2* seg_bounds, uint64_t* keys, uint32_t* idx, uint32_t* hist,
                    int n_seg_passes, cudaStream_t st);
 
+// Bounds, encode and sort of one segment of up to kFrontMax particles in one
+// launch (k_front.cu): the sorted keys and positions.  front_available: the
+// current device runs its clusters.
+// Whole step in us, separate stages / one launch, plain launches and graph:
+//    1,408 particles  188 / 136  and 154 / 123
+//    8,192            228 / 176      194 / 168
+//   32,768            321 / 287      290 / 281
+//   45,056            354 / 324      320 / 317
+//   65,536            413 / 400      380 / 392
+constexpr int kFrontMax = 49152;
+constexpr int kFrontBoundsReduce = 0;  // reduce the bounds, and write seg_bounds
+constexpr int kFrontBoundsGiven = 1;   // read seg_bounds
+constexpr int kFrontBoundsCaller = 2;  // gmin, gmax
+bool front_available();
+void launch_front(const float4* pos, int n, int front_bounds, float gmin, float gmax, float2* seg_bounds,
+                  uint64_t* keys, uint32_t* idx, uint32_t* status, cudaStream_t st);
+
 size_t sort_lookback_words(int64_t n, int passes);
 size_t sort_lookback_words_upto(int64_t n, int passes);  // the most any m <= n needs
 void launch_sort_pass(const Layout& L, int pass, const uint64_t* keys_in, const uint32_t* vals_in,
