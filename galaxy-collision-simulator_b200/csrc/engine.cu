@@ -83,9 +83,6 @@ struct gcs_ctx {
     // the sort); the build stage joins it
     cudaEvent_t gather_fork = nullptr, gather_join = nullptr;
     bool gather_pending = false;
-    float4* split_sums = nullptr;         // parts of split walk groups: 32 sums per unit
-    bool split_any = false;               // whether the unit table holds parts of split groups
-    uint32_t* split_arrived = nullptr;    // parts arrived, per group (zero between walks)
     std::vector<int32_t> h_group_super;   // super-group of each walk group (host copy)
     Chunk* chunks = nullptr;
     float2* seg_bounds = nullptr;
@@ -291,7 +288,7 @@ void free_all(gcs_ctx* c) {
     if (c->host_copy) HostCopy::release();
     void* ptrs[] = {c->pos[0], c->pos[1], c->vel[0], c->vel[1], c->acc, c->keys[0], c->keys[1],
                     c->idx[0], c->idx[1], c->tr, c->bd, c->wn, c->com64, c->leaf_parent, c->seg_off,
-                    c->seg_id, c->groups, c->supers, c->sg_list, c->sg_src, c->sg_meta, c->perm, c->split_sums, c->split_arrived, c->chunks,
+                    c->seg_id, c->groups, c->supers, c->sg_list, c->sg_src, c->sg_meta, c->perm, c->chunks,
                     c->seg_bounds, c->staging, c->pb_staging,
                     c->scratch, c->status, c->diag, c->targets, c->direct_out, c->direct_sums, c->counts,
                     c->walk_stack, c->render_acc, c->render_rgba, c->star_chunk_done};
@@ -351,37 +348,6 @@ int split_levels(int width) {
     return (kSuperTargets >> levels) == width ? levels : 0;
 }
 
-// Walk units a group is split into, by its segment's size alone (so that a
-// segment's sums are the same bits alone and beside others).  A segment of
-// up to about 150,000 particles has fewer 32-target groups than the chip has
-// walk warps (4,736), and the walk takes as long as its longest group.  Each
-// part adds a tail of small rounds (one per tree level), which large
-// segments would only pay for.  Walk stage in us at theta 0.5, leaf 8, by
-// parts 1 / 2 / 4 / 8 (CUDA events):
-//     8,192 particles   176 / 127 / 119 /  92
-//    16,384             201 / 150 / 150 / 139
-//    45,056             297 / 225 / 199 / 229     (theta 0.7: 172 / 150 / 133 / 162)
-//    90,000             391 / 313 / 313 / 365
-//   131,072             484 / 424 / 428 / 516     (theta 0.7: 297 / 258 / 266 / 305)
-//   262,144             743 / 715 / 793 / 973
-//   1,048,576 (leaf 4) 2403 /2455 /2860 /3638
-// Other group widths are never split (wider groups run two targets a lane,
-// narrower ones already have twice the groups).
-constexpr int kSplitWidth = 32;
-constexpr int64_t kSplit8Max = 24 * 1024, kSplit4Max = 64 * 1024, kSplit2Max = 160 * 1024;
-int walk_parts(int64_t n, int width) {
-    if (width != kSplitWidth) return 1;
-    return n <= kSplit8Max ? 8 : n <= kSplit4Max ? 4 : n <= kSplit2Max ? 2 : 1;
-}
-
-// The most units any layout of at most n particles in at most `segments`
-// segments gives kSplitWidth-target groups.
-size_t split_units(size_t n, int32_t segments) {
-    constexpr size_t per_segment = std::max({kSplit8Max * 8, kSplit4Max * 4, kSplit2Max * 2}) / kSplitWidth;
-    return std::min(n / kSplitWidth * 8 + 8 * (size_t)segments,
-                    n / kSplitWidth + (per_segment + 1) * (size_t)segments);
-}
-
 // Whether the walk takes its targets through a partition of each super-group.
 bool partitioned(const gcs_ctx* c) { return c->walk_frontier && split_levels(c->group_width) > 0; }
 
@@ -401,7 +367,6 @@ int upload_groups(gcs_ctx* c) {
     std::vector<WalkGroup> groups;
     std::vector<SuperGroup> supers;
     groups.reserve((size_t)(c->n / c->group_width + c->nseg + 1));
-    bool any_split = false;
     const int64_t rf = range_first(c), rl = rf + range_count(c);
     // Super-groups are aligned to the segment start and always cover all of
     // their targets, also where a step range cuts one: its box, and so its
@@ -412,12 +377,11 @@ int upload_groups(gcs_ctx* c) {
     for (int s = 0; s < c->nseg; ++s) {
         const int64_t a = c->h_seg_off[s], e = c->h_seg_off[s + 1];
         int64_t cur = -1;  // first target of the current super-group
-        const int parts = walk_parts(e - a, c->group_width);
         for (int64_t g = a; g < e; g += c->group_width) {
             if (g < rf || g >= rl) continue;  // outside this context's step range
             WalkGroup w;
             w.start = (int32_t)g;
-            const int32_t count = (int32_t)std::min<int64_t>(c->group_width, e - g);
+            w.count = (int32_t)std::min<int64_t>(c->group_width, e - g);
             w.seg = s;
             const int64_t sg_first = a + (g - a) / span * span;
             if (sg_first != cur) {
@@ -430,11 +394,7 @@ int upload_groups(gcs_ctx* c) {
                 cur = sg_first;
             }
             w.super = (int32_t)supers.size() - 1;
-            any_split |= parts > 1;
-            for (int part = 0; part < parts; ++part) {
-                w.packed = count | part << 8 | parts << 16;
-                groups.push_back(w);
-            }
+            groups.push_back(w);
         }
     }
     if (groups.size() > c->groups_cap || supers.size() > c->supers_cap) {
@@ -450,7 +410,6 @@ int upload_groups(gcs_ctx* c) {
                                     cudaMemcpyHostToDevice, c->stream));
     c->n_supers = (int)supers.size();
     c->n_groups = (int)groups.size();
-    c->split_any = any_split;
     c->h_group_super.resize(groups.size());
     for (size_t g = 0; g < groups.size(); ++g) c->h_group_super[g] = groups[g].super;
     c->h_group_start.resize(groups.size());
@@ -535,13 +494,9 @@ static int walk_stage(gcs_ctx* c, const gcs_params* p, const WalkEpilogue& ep) {
         fr.fork = c->part_fork;
         fr.join = c->part_join;
     }
-    WalkSplit split;
-    split.sums = c->split_sums;
-    split.arrived = c->split_arrived;
-    split.any = c->split_any;
     launch_walk(L, wp, c->pos[c->cur], c->wn, c->groups, c->n_groups, c->group_width > 32 ? 2 : 1, c->acc,
                 scratch_at<uint32_t>(c, sl.walk_q), c->status, p->walk_blocks_per_sm, c->sm_count,
-                c->count_walk ? c->counts : nullptr, c->walk_stack, c->walk_stack_entries, st, split, ep, fr);
+                c->count_walk ? c->counts : nullptr, c->walk_stack, c->walk_stack_entries, st, ep, fr);
     return check_launch(c, "walk");
 }
 
@@ -765,7 +720,6 @@ int gcs_create(gcs_ctx** out, int64_t capacity, int32_t max_segments, int32_t de
     c->front = front_available();
     cudaMemset(c->scratch, 0, c->scratch_cap);  // the walk queue starts (and stays) at zero
     cudaMemset(c->status, 0, sizeof(uint32_t));
-    cudaMemset(c->split_arrived, 0, sizeof(uint32_t) * split_units((size_t)capacity, max_segments));
     cudaMemset(c->wn, 0, sizeof(WalkNode) * (size_t)capacity);  // codes of unwritten records stay in range
     cudaMemset(c->acc, 0, sizeof(float4) * (size_t)capacity);
     int64_t cnt = capacity;
@@ -807,8 +761,7 @@ static int allocate_state(gcs_ctx* c) {
     const int32_t max_segments = c->max_segments;
     const size_t N = (size_t)capacity;
     // groups as narrow as kMinGroupWidth targets (the autotuner's smallest)
-    // and the units of split 32-target groups
-    const size_t max_groups = std::max(N / kMinGroupWidth + (size_t)max_segments, split_units(N, max_segments)) + 1;
+    const size_t max_groups = N / kMinGroupWidth + (size_t)max_segments + 1;
     c->groups_cap = max_groups;
     const size_t max_chunks = N / kChunkSize + (size_t)max_segments + 1;
     int rc = GCS_OK;
@@ -827,8 +780,6 @@ static int allocate_state(gcs_ctx* c) {
     if (!rc) rc |= dalloc(c, &c->seg_off, (size_t)max_segments + 1);
     if (!rc) rc |= dalloc(c, &c->seg_id, N);
     if (!rc) rc |= dalloc(c, &c->groups, max_groups);
-    if (!rc) rc |= dalloc(c, &c->split_sums, split_units(N, max_segments) * 32);
-    if (!rc) rc |= dalloc(c, &c->split_arrived, split_units(N, max_segments));
     // super-groups: full ones hold more than kSuperTargets - kGroupSize
     // targets; a segment (or a step range within it) ends at most one
     // partial one
@@ -1298,9 +1249,8 @@ static int step_host_overlapped(gcs_ctx* c, const gcs_params* p, Star* host, int
     bound.push_back(0);
     const bool snap = partitioned(c);
     auto add_bound = [&](int g) {
-        // (nor between the parts of one group)
-        const std::vector<int32_t>& edge = snap ? c->h_group_super : c->h_group_start;
-        while (g < ng && g > 0 && edge[(size_t)g] == edge[(size_t)g - 1]) ++g;
+        if (snap)
+            while (g < ng && g > 0 && c->h_group_super[(size_t)g] == c->h_group_super[(size_t)g - 1]) ++g;
         if (g > bound.back()) bound.push_back(g);
     };
     for (int g = hpc; g < head_groups; g += hpc) add_bound(g);

@@ -68,18 +68,13 @@ constexpr int kLookGroup = 16;      // tiles per look-back group
 constexpr int kGroupSize = 64;         // walk targets per warp group (two per lane above 32)
 
 // Work unit of the walk: up to kGroupSize consecutive sorted particles of one
-// segment; `super` is its super-group (walk frontiers, below).  A group of a
-// small segment is split into `parts` units (walk_parts), consecutive in the
-// table, that share its targets and divide its super-group's lists.
+// segment; `super` is its super-group (walk frontiers, below).
 struct WalkGroup {
     int32_t start;
-    int32_t packed;  // count | part << 8 | parts << 16
+    int32_t count;
     int32_t seg;
     int32_t super;
 };
-__host__ __device__ inline int group_count(const WalkGroup& g) { return g.packed & 0xFF; }
-__host__ __device__ inline int group_part(const WalkGroup& g) { return (g.packed >> 8) & 0xFF; }
-__host__ __device__ inline int group_parts(const WalkGroup& g) { return g.packed >> 16; }
 
 // Per-segment bounds chunk: a range of particles of one segment.
 struct Chunk {
@@ -260,7 +255,7 @@ constexpr int kWalkBlockWarps = 8;  // warps per walk block
 // invalid and its groups walk from the root.
 constexpr int kSuperTargets = 256;
 constexpr int kSuperCap = 2048;     // take nodes (from the front) + frontier nodes (from the back)
-constexpr int kSuperSrcCap = 1024;  // particle sources of a super-group (leaf 8 at 16,384 particles: up to 284)
+constexpr int kSuperSrcCap = 256;   // particle sources of a super-group
 // Targets [start, start + count) of segment seg (a run of whole groups).
 struct SuperGroup {
     int32_t start;
@@ -289,20 +284,11 @@ struct WalkFrontier {
     cudaEvent_t fork = nullptr, join = nullptr;
 };
 
-// Sums of the parts of split groups: a row of 32 targets per unit, and per
-// group (at its first unit) the number of parts that have arrived; the
-// counters are zero between launches.
-struct WalkSplit {
-    float4* sums = nullptr;
-    uint32_t* arrived = nullptr;
-    bool any = false;  // whether the table holds parts (only units of 32-target groups may be)
-};
-
 void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
                  const WalkNode* wn, const WalkGroup* groups, int n_groups, int targets_per_lane,
                  float4* acc, uint32_t* queue, uint32_t* status, int blocks_per_sm,
                  int sm_count, unsigned long long* counts, int2* gstack, size_t gstack_entries,
-                 cudaStream_t st, const WalkSplit& split, const WalkEpilogue& ep = WalkEpilogue(),
+                 cudaStream_t st, const WalkEpilogue& ep = WalkEpilogue(),
                  const WalkFrontier& fr = WalkFrontier());
 int walk_max_blocks_per_sm(int batch, int with_potential, int targets_per_lane);
 // Persistent walk grid (blocks) for n_groups groups, and the global stack

@@ -51,11 +51,6 @@
 // stops with GCS_DEV_TREE_MALFORMED.  The work queue resets itself: the last
 // warp to find it empty zeroes it.
 //
-// Small segments have too few groups to fill the chip: their groups come as
-// several units (WalkSplit) that each take a share of the super-group's take
-// list, sources and frontier; the unit that arrives last adds the parts'
-// sums in part order (45,056 particles, 4 parts: walk stage 297 -> 199 us).
-//
 // With an epilogue (WalkEpilogue), a warp that has written its group's
 // accelerations also applies the step's kick/drift to those particles, out of
 // place, and writes their Star records (when given); the warp that completes a chunk of
@@ -68,7 +63,6 @@
 // go straight into it and no chunk is counted (host_flags == nullptr).
 #include <algorithm>
 #include <atomic>
-#include <type_traits>
 
 #include "gcs_internal.h"
 #include "device_math.cuh"
@@ -336,15 +330,14 @@ __device__ __forceinline__ uint32_t warp_exclusive_scan(uint32_t v, int lane) {
     return x - v;
 }
 
-// kSplit: some unit of the launch is a part of a split group (T = 1).
-template <int H, int T, bool kPot, bool kCount, bool kSplit>
+template <int H, int T, bool kPot, bool kCount>
 __global__ void __launch_bounds__(kWalkThreads, (WalkOcc<H, T>::kMinBlocks))
 walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
             const WalkNode* __restrict__ wn, const WalkGroup* __restrict__ groups,
             int n_groups, float4* __restrict__ acc, uint32_t* __restrict__ queue,
             uint32_t* __restrict__ status, unsigned long long* __restrict__ counts,
             typename EntryOf<T>::type* __restrict__ gstack, int gstack_cap, WalkEpilogue ep,
-            WalkFrontier fr, WalkSplit split) {
+            WalkFrontier fr) {
     using Smem = WarpSmem<H, T>;
     using Entry = typename Smem::Entry;
     extern __shared__ __align__(16) unsigned char walk_smem[];
@@ -368,8 +361,6 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
         g = __shfl_sync(kFull, g, 0);
         if (g >= n_groups) break;
         const WalkGroup grp = groups[g];
-        const int grp_count = group_count(grp), part = kSplit ? group_part(grp) : 0,
-                  parts = kSplit ? group_parts(grp) : 1;
         bool valid[T];
         uint32_t live[T];
         Targets<T> X;
@@ -379,7 +370,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
         Accum A[T];
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            valid[t] = lane + 32 * t < grp_count;
+            valid[t] = lane + 32 * t < grp.count;
             float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
             if (valid[t]) {
                 const int j = grp.start + lane + 32 * t;
@@ -421,12 +412,10 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
             if (fm.w && fm.z - Smem::kSpillAbove <= gstack_cap) {
                 // the super-group's shared work: its take list for every
                 // target (two records per lane per chunk of 64, staged in the
-                // source pairs), its sources, then the frontier as the stack;
-                // a part of a split group takes its share of each
+                // source pairs), its sources, then the frontier as the stack
                 const int32_t* tl = fr.list + (size_t)grp.super * kSuperCap;
-                const int t_end = fm.x * (part + 1) / parts;
-                for (int base = fm.x * part / parts; base < t_end; base += kSrcCap) {
-                    const int cnt = min(kSrcCap, t_end - base);
+                for (int base = 0; base < fm.x; base += kSrcCap) {
+                    const int cnt = min(kSrcCap, fm.x - base);
                     const int padded = (cnt + 1) & ~1;
                     for (int e = lane; e < padded; e += 32) {
                         float4 q = make_float4(1e30f, 1e30f, 1e30f, 0.0f);
@@ -447,18 +436,16 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                     __syncwarp();
                 }
                 if (kCount) {
-                    const uint32_t n_list = (uint32_t)(t_end - fm.x * part / parts);
 #pragma unroll
                     for (int t = 0; t < T; ++t)
-                        if (valid[t]) A[t].n_mono += n_list;
-                    WC.w_node += n_list;
-                    WC.all_take += n_list;
-                    WC.r_list += n_list;
+                        if (valid[t]) A[t].n_mono += (uint32_t)fm.x;
+                    WC.w_node += (uint32_t)fm.x;
+                    WC.all_take += (uint32_t)fm.x;
+                    WC.r_list += (uint32_t)fm.x;
                 }
                 const int32_t* sl = fr.src + (size_t)grp.super * kSuperSrcCap;
-                const int s_end = fm.y * (part + 1) / parts;
-                for (int base = fm.y * part / parts; base < s_end; base += kSrcCap) {
-                    const int cnt = min(kSrcCap, s_end - base);
+                for (int base = 0; base < fm.y; base += kSrcCap) {
+                    const int cnt = min(kSrcCap, fm.y - base);
                     for (int e = lane; e < cnt; e += 32) {
                         W.srcp[e] = __ldg(sl + base + e);
 #pragma unroll
@@ -468,17 +455,13 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                 }
                 // frontier entries [kSuperCap - n_front, kSuperCap): what the
                 // shared stack cannot hold goes to the global bottom
-                // (of a split group, every parts-th entry: neighbours in the
-                // list are siblings with subtrees of like size)
-                const int32_t* fl = tl + kSuperCap - fm.z + part;
-                const int n_front = (fm.z - part + parts - 1) / parts;
-                const int to_g = max(0, n_front - Smem::kSpillAbove);
-                for (int j = lane; j < to_g; j += 32) gstk[j] = make_entry(__ldg(fl + j * parts), live);
-                for (int j = lane; j < n_front - to_g; j += 32)
-                    W.stk[j] = make_entry(__ldg(fl + (to_g + j) * parts), live);
+                const int32_t* fl = tl + kSuperCap - fm.z;
+                const int to_g = max(0, fm.z - Smem::kSpillAbove);
+                for (int j = lane; j < to_g; j += 32) gstk[j] = make_entry(__ldg(fl + j), live);
+                for (int j = lane; j < fm.z - to_g; j += 32) W.stk[j] = make_entry(__ldg(fl + to_g + j), live);
                 gtop = to_g;
-                top = n_front - to_g;
-            } else if (part == 0) {  // no lists: the first part walks from the root
+                top = fm.z - to_g;
+            } else {
                 if (lane == 0) W.stk[0] = make_entry(off - s, live);
                 top = 1;
             }
@@ -800,47 +783,13 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
             }
         }
         if (nsrc > 0) flush_sources<H, T, kPot, kCount>(W, nsrc, lane, lane_bit, pos, G, X, e2, leaf_thr, A, WC);
-        // a part of a split group leaves its sums; the part that arrives last
-        // adds all of them in part order and finishes the group (so the
-        // result does not depend on which part that is)
-        // (the unit's record is read again: nothing of it is held over the walk)
-        const WalkGroup unit = groups[g];
-        const int n_parts = kSplit ? group_parts(unit) : 1;
-        const int first = g - (kSplit ? group_part(unit) : 0);
-        bool finish = true;
-        if (kSplit && n_parts > 1) {
-            split.sums[(size_t)g * 32 + lane] =
-                make_float4(__fadd_rn(A[0].ax.x, A[0].ax.y), __fadd_rn(A[0].ay.x, A[0].ay.y),
-                            __fadd_rn(A[0].az.x, A[0].az.y), __fadd_rn(A[0].pot.x, A[0].pot.y));
-            __threadfence();
-            __syncwarp();
-            uint32_t before = 0;
-            if (lane == 0) before = atomicAdd(split.arrived + first, 1u);
-            before = __shfl_sync(kFull, before, 0);
-            finish = before == (uint32_t)n_parts - 1u;
-            if (finish) {
-                __threadfence();
-                if (lane == 0) split.arrived[first] = 0u;
-            }
-        }
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            if (!finish || lane + 32 * t >= group_count(unit)) continue;
-            const int j = unit.start + lane + 32 * t;
+            if (!valid[t]) continue;
+            const int j = grp.start + lane + 32 * t;
             const int64_t i = fr.perm ? __ldg(fr.perm + j) : j;  // the target's particle
-            float4 a;
-            if (kSplit && n_parts > 1) {
-                const float4* rows = split.sums + (size_t)first * 32 + lane;
-                a = __ldcg(rows);
-                for (int q = 1; q < n_parts; ++q) {
-                    const float4 b = __ldcg(rows + 32 * q);
-                    a = make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z),
-                                    __fadd_rn(a.w, b.w));
-                }
-            } else {
-                a = make_float4(__fadd_rn(A[t].ax.x, A[t].ax.y), __fadd_rn(A[t].ay.x, A[t].ay.y),
-                                __fadd_rn(A[t].az.x, A[t].az.y), __fadd_rn(A[t].pot.x, A[t].pot.y));
-            }
+            const float4 a = make_float4(__fadd_rn(A[t].ax.x, A[t].ax.y), __fadd_rn(A[t].ay.x, A[t].ay.y),
+                                         __fadd_rn(A[t].az.x, A[t].az.y), __fadd_rn(A[t].pot.x, A[t].pot.y));
             acc[i] = a;
             if (ep.vel_in) {
                 // the step's kick/drift of this target, out of place, and its Star
@@ -1172,20 +1121,20 @@ constexpr size_t smem_bytes() {
 
 // Opt the instantiation in to its dynamic shared memory (above 48 KB), once
 // per device.
-template <int H, int T, bool kPot, bool kCount, bool kSplit>
+template <int H, int T, bool kPot, bool kCount>
 void configure() {
     static std::once_flag done[kMaxDevices];
     once_per_device(done, [] {
-        cudaFuncSetAttribute(walk_kernel<H, T, kPot, kCount, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(walk_kernel<H, T, kPot, kCount>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem_bytes<H, T>());
     });
 }
 
 template <int H, int T, bool kPot, bool kCount>
 int occupancy_of() {
-    configure<H, T, kPot, kCount, false>();
+    configure<H, T, kPot, kCount>();
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, walk_kernel<H, T, kPot, kCount, false>, kWalkThreads,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, walk_kernel<H, T, kPot, kCount>, kWalkThreads,
                                                   smem_bytes<H, T>());
     return nb > 0 ? nb : 1;
 }
@@ -1229,27 +1178,32 @@ size_t walk_stack_entries(int64_t grid_blocks) {
     return (size_t)grid_blocks * kWalkWarps * (size_t)kWalkGlobalStack;
 }
 
-template <int H, int T, bool kSplit>
+template <int H, int T>
 static void launch_ht(const Layout& L, const WalkParams& q, const float4* pos, const WalkNode* wn,
                       const WalkGroup* groups, int n_groups, float4* acc, uint32_t* queue, uint32_t* status,
                       unsigned long long* counts, int2* gstack, int cap, unsigned g, cudaStream_t st,
-                      const WalkEpilogue& ep, const WalkFrontier& fr, const WalkSplit& split) {
+                      const WalkEpilogue& ep, const WalkFrontier& fr) {
     using Entry = typename EntryOf<T>::type;
     Entry* gs = reinterpret_cast<Entry*>(gstack);
     const size_t sm = smem_bytes<H, T>();
-    const auto go = [&](auto pot, auto count) {
-        constexpr bool kPot = decltype(pot)::value, kCount = decltype(count)::value;
-        configure<H, T, kPot, kCount, kSplit>();
-        walk_kernel<H, T, kPot, kCount, kSplit><<<g, kWalkThreads, sm, st>>>(
-            L, q, pos, wn, groups, n_groups, acc, queue, status, kCount ? counts : nullptr, gs, cap, ep, fr, split);
-    };
     if (counts) {
-        if (q.with_potential) go(std::true_type{}, std::true_type{});
-        else go(std::false_type{}, std::true_type{});
+        if (q.with_potential) {
+            configure<H, T, true, true>();
+            walk_kernel<H, T, true, true><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue,
+                                                                       status, counts, gs, cap, ep, fr);
+        } else {
+            configure<H, T, false, true>();
+            walk_kernel<H, T, false, true><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue,
+                                                                        status, counts, gs, cap, ep, fr);
+        }
     } else if (q.with_potential) {
-        go(std::true_type{}, std::false_type{});
+        configure<H, T, true, false>();
+        walk_kernel<H, T, true, false><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue,
+                                                                    status, nullptr, gs, cap, ep, fr);
     } else {
-        go(std::false_type{}, std::false_type{});
+        configure<H, T, false, false>();
+        walk_kernel<H, T, false, false><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue,
+                                                                     status, nullptr, gs, cap, ep, fr);
     }
 }
 
@@ -1257,7 +1211,7 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
                  const WalkNode* wn, const WalkGroup* groups, int n_groups, int targets_per_lane, float4* acc,
                  uint32_t* queue, uint32_t* status, int blocks_per_sm, int sm_count,
                  unsigned long long* counts, int2* gstack, size_t gstack_entries, cudaStream_t st,
-                 const WalkSplit& split, const WalkEpilogue& ep, const WalkFrontier& fr_in) {
+                 const WalkEpilogue& ep, const WalkFrontier& fr_in) {
     if (n_groups <= 0) return;
     WalkFrontier fr = fr_in;
     if (fr.supers && fr.n_supers > 0 && fr.list && fr.src && fr.meta) {
@@ -1305,22 +1259,15 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
     // entries per warp region: the whole buffer split over this grid's warps
     const size_t units = gstack_entries / ((size_t)grid * kWalkWarps);
     const int cap = (int)(std::min<size_t>(units, (size_t)1 << 24) / (size_t)T);
-    const auto go = [&](auto h, auto t, auto any_split) {
-        launch_ht<decltype(h)::value, decltype(t)::value, decltype(any_split)::value>(
-            L, q, pos, wn, groups, n_groups, acc, queue, status, counts, gstack, cap, g, st, ep, fr, split);
-    };
-    const std::integral_constant<int, 1> one{};
-    const std::integral_constant<int, 2> two{};
     if (T == 2) {
-        if (q.batch > 32) go(two, two, std::false_type{});
-        else go(one, two, std::false_type{});
-    } else if (split.any) {
-        if (q.batch > 32) go(two, one, std::true_type{});
-        else go(one, one, std::true_type{});
+        if (q.batch > 32)
+            launch_ht<2, 2>(L, q, pos, wn, groups, n_groups, acc, queue, status, counts, gstack, cap, g, st, ep, fr);
+        else
+            launch_ht<1, 2>(L, q, pos, wn, groups, n_groups, acc, queue, status, counts, gstack, cap, g, st, ep, fr);
     } else if (q.batch > 32) {
-        go(two, one, std::false_type{});
+        launch_ht<2, 1>(L, q, pos, wn, groups, n_groups, acc, queue, status, counts, gstack, cap, g, st, ep, fr);
     } else {
-        go(one, one, std::false_type{});
+        launch_ht<1, 1>(L, q, pos, wn, groups, n_groups, acc, queue, status, counts, gstack, cap, g, st, ep, fr);
     }
 }
 
