@@ -255,7 +255,7 @@ constexpr int kWalkBlockWarps = 8;  // warps per walk block
 // invalid and its groups walk from the root.
 constexpr int kSuperTargets = 256;
 constexpr int kSuperCap = 2048;     // take nodes (from the front) + frontier nodes (from the back)
-constexpr int kSuperSrcCap = 256;   // particle sources of a super-group
+constexpr int kSuperSrcCap = 1024;  // particle sources of a super-group (leaf 8 at 16,384 particles: up to 284)
 // Targets [start, start + count) of segment seg (a run of whole groups).
 struct SuperGroup {
     int32_t start;

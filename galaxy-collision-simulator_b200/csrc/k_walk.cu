@@ -51,6 +51,9 @@
 // stops with GCS_DEV_TREE_MALFORMED.  The work queue resets itself: the last
 // warp to find it empty zeroes it.
 //
+// With few groups two warps walk each one together, with the same rounds and
+// the same sums (walk_pair_kernel).
+//
 // With an epilogue (WalkEpilogue), a warp that has written its group's
 // accelerations also applies the step's kick/drift to those particles, out of
 // place, and writes their Star records (when given); the warp that completes a chunk of
@@ -328,6 +331,40 @@ __device__ __forceinline__ uint32_t warp_exclusive_scan(uint32_t v, int lane) {
         if (lane >= o) x += y;
     }
     return x - v;
+}
+
+// A target's acceleration, and with an epilogue the step's kick/drift of its
+// particle i, out of place, and its Star.
+__device__ __forceinline__ void finish_target(const float4* __restrict__ pos, float4* __restrict__ acc,
+                                              const WalkEpilogue& ep, int64_t i, float4 a) {
+    acc[i] = a;
+    if (ep.vel_in) {
+        float4 p = __ldg(pos + i);
+        float4 v = __ldg(ep.vel_in + i);
+        kick_drift(p, v, a, ep.dt, ep.recolor);
+        ep.pos_out[i] = p;
+        ep.vel_out[i] = v;
+        if (ep.stars) store_star(ep.stars, i, p, v);
+    }
+}
+// Count a finished group in its chunk (one lane, after its warp's stores); the
+// one that completes the chunk tells the host (every group fences before
+// counting, so a chunk seen complete has all of its records written).
+__device__ __forceinline__ void finish_group(const WalkEpilogue& ep, int g) {
+    __threadfence();
+    // the chunk holding group g: the last boundary <= g
+    int lo = 0, hi = ep.n_chunks - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (ep.chunk_bound[mid] <= g) lo = mid;
+        else hi = mid - 1;
+    }
+    const int k = lo;
+    const int in_chunk = ep.chunk_bound[k + 1] - ep.chunk_bound[k];
+    if (atomicAdd(ep.chunk_done + k, 1u) == (uint32_t)in_chunk - 1u) {
+        __threadfence_system();
+        *reinterpret_cast<volatile uint32_t*>(ep.host_flags + k) = ep.epoch;
+    }
 }
 
 template <int H, int T, bool kPot, bool kCount>
@@ -790,38 +827,11 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
             const int64_t i = fr.perm ? __ldg(fr.perm + j) : j;  // the target's particle
             const float4 a = make_float4(__fadd_rn(A[t].ax.x, A[t].ax.y), __fadd_rn(A[t].ay.x, A[t].ay.y),
                                          __fadd_rn(A[t].az.x, A[t].az.y), __fadd_rn(A[t].pot.x, A[t].pot.y));
-            acc[i] = a;
-            if (ep.vel_in) {
-                // the step's kick/drift of this target, out of place, and its Star
-                float4 p = __ldg(pos + i);
-                float4 v = __ldg(ep.vel_in + i);
-                kick_drift(p, v, a, ep.dt, ep.recolor);
-                ep.pos_out[i] = p;
-                ep.vel_out[i] = v;
-                if (ep.stars) store_star(ep.stars, i, p, v);
-            }
+            finish_target(pos, acc, ep, i, a);
         }
         if (ep.vel_in && ep.host_flags) {
-            // count the group in its chunk; the warp that completes the chunk
-            // tells the host (every warp fences before counting, so a chunk
-            // seen complete has all of its records written)
             __syncwarp();
-            if (lane == 0) {
-                __threadfence();
-                // the chunk holding group g: the last boundary <= g
-                int lo = 0, hi = ep.n_chunks - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (ep.chunk_bound[mid] <= g) lo = mid;
-                    else hi = mid - 1;
-                }
-                const int k = lo;
-                const int in_chunk = ep.chunk_bound[k + 1] - ep.chunk_bound[k];
-                if (atomicAdd(ep.chunk_done + k, 1u) == (uint32_t)in_chunk - 1u) {
-                    __threadfence_system();
-                    *reinterpret_cast<volatile uint32_t*>(ep.host_flags + k) = ep.epoch;
-                }
-            }
+            if (lane == 0) finish_group(ep, g);
         }
         if (kCount) {
             unsigned long long cm = 0ull, cp = 0ull;
@@ -857,6 +867,460 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
     // last of them knows no warp will touch the queue again and resets it.
     if (lane == 0) {
         const uint32_t total = gridDim.x * kWalkWarps;
+        if (atomicAdd(queue + 1, 1u) == total - 1) {
+            queue[0] = 0u;
+            queue[1] = 0u;
+            __threadfence();
+        }
+    }
+}
+
+// ---- the walk of a group by two warps -------------------------------------------
+// With fewer groups than the chip has walk warps the walk takes as long as
+// its longest group, and a group is one serial chain of rounds of one warp.
+// Here two warps of a block walk one group together, on the same lists in
+// shared memory: each fetches, classifies and expands one half of a round's
+// nodes (the h = 0 and h = 1 nodes of the one-warp kernel), and each evaluates
+// every other slot of the evaluation lists for all targets: warp w takes the
+// slots of parity w, whose terms the one-warp kernel adds to the w-th of its
+// two partial sums.  Rounds, lists and every partial sum are those of the
+// one-warp kernel, so the results are its bits, and which kernel runs can go
+// by how many groups the whole context has.
+//
+// Two slots of a warp's parity are evaluated at once (packed FP32) and added
+// one after the other.  List slot s is pair (s >> 2), element (s >> 1) & 1 of
+// half s & 1; a list takes whole pairs in both halves, unused entries are
+// empty (mass 0 at 1e30, masks 0) and add nothing.
+template <int H>
+struct PairSmem {
+    static constexpr int kBatch = 32 * H;
+    static constexpr int kStackCap = WarpSmem<H, 1>::kStackCap;
+    static constexpr int kSpillAbove = WarpSmem<H, 1>::kSpillAbove;
+    static constexpr int kPairs = kBatch / 4 + 3;  // of one half: three lists of whole pairs
+    int2 stk[kStackCap];
+    struct Half {
+        float4 xy[kPairs], zm[kPairs];
+        float2 w2[kPairs];
+        uint2 mask[kPairs], nopen[kPairs];
+        float4 sxy[kSrcCap / 4], szm[kSrcCap / 4];
+        uint2 smask[kSrcCap / 4];
+    } half[2];
+    int4 sdesc[kBatch];
+    uint32_t dmask[kBatch];
+    int srcp[kSrcCap];
+    uint32_t srcm[kSrcCap];
+    uint32_t ball[2][3];
+    uint32_t cnt[2][32];
+    float4 sums[32];
+    int item;
+};
+constexpr int kPairBlockPairs = kWalkWarps / 2;
+// Three blocks (80 registers, no spills) against four (64) and two (128):
+// 60,000 particles at theta 0.7 139, 156 and 160 us, 16,384 at 0.5 135, 141
+// and 131.
+constexpr int kPairMinBlocks = 3;
+
+// Barrier of the two warps of pair `id` of the block.
+__device__ __forceinline__ void pair_sync(int id) {
+    asm volatile("bar.sync %0, 64;" :: "r"(id + 1) : "memory");
+}
+
+// Entry e of a float4 pair array: element (e & 1) of pair (e >> 1).
+__device__ __forceinline__ void put_entry(float4* xy, float4* zm, int e, float4 c) { put_pair(xy, zm, e, c); }
+
+struct Half2Sums {
+    float ax, ay, az, pot;
+};
+// The terms of two slots, one after the other, into the warp's partial sums
+// (pair_add's arithmetic).
+template <bool kPot>
+__device__ __forceinline__ void half_add(Half2Sums& A, const PairD& d, float4 zm, bool use0, bool use1) {
+    const float2 inv = make_float2(rsqrt_approx(d.d2.x), rsqrt_approx(d.d2.y));
+    const float2 inv3 = __fmul2_rn(__fmul2_rn(inv, inv), inv);
+    float2 f = __fmul2_rn(make_float2(zm.z, zm.w), inv3);
+    f.x = use0 ? f.x : 0.0f;
+    f.y = use1 ? f.y : 0.0f;
+    A.ax = __fmaf_rn(d.dx.y, f.y, __fmaf_rn(d.dx.x, f.x, A.ax));
+    A.ay = __fmaf_rn(d.dy.y, f.y, __fmaf_rn(d.dy.x, f.x, A.ay));
+    A.az = __fmaf_rn(d.dz.y, f.y, __fmaf_rn(d.dz.x, f.x, A.az));
+    if (kPot) {
+        A.pot = use0 ? __fmaf_rn(-zm.z, inv.x, A.pot) : A.pot;
+        A.pot = use1 ? __fmaf_rn(-zm.w, inv.y, A.pot) : A.pot;
+    }
+}
+
+// flush_sources for a pair of warps.
+template <int H, bool kPot>
+__device__ __forceinline__ void flush_pair(PairSmem<H>& W, int nsrc, int id, int w, int lane, uint32_t lane_bit,
+                                           const float4* __restrict__ pos, float G, const Targets<1>& X, float2 e2,
+                                           float leaf_thr, Half2Sums& A) {
+    pair_sync(id);  // the list is complete
+    const int slots = (nsrc + 3) & ~3;
+    for (int e = lane + 32 * w; e < slots; e += 64) {
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t m = 0u;
+        if (e < nsrc) {
+            q = __ldg(pos + W.srcp[e]);
+            q.w = __fmul_rn(G, q.w);
+            m = W.srcm[e];
+        }
+        auto& S = W.half[e & 1];
+        put_entry(S.sxy, S.szm, e >> 1, q);
+        put_mask(S.smask, e >> 1, m);
+    }
+    pair_sync(id);
+    const auto& S = W.half[w];
+#pragma unroll 4
+    for (int q = 0; q < (slots >> 2); ++q) {
+        const float4 zm = S.szm[q];
+        const float4 xy = S.sxy[q];
+        const uint2 mk = S.smask[q];
+        const PairD d = pair_d(xy, zm, X.npx[0], X.npy[0], X.npz[0], e2);
+        half_add<kPot>(A, d, zm, (mk.x & lane_bit) && (d.d2.x > leaf_thr), (mk.y & lane_bit) && (d.d2.y > leaf_thr));
+    }
+    pair_sync(id);  // the list may be written again
+}
+
+template <int H, bool kPot>
+__global__ void __launch_bounds__(kWalkThreads, kPairMinBlocks)
+walk_pair_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos, const WalkNode* __restrict__ wn,
+                 const WalkGroup* __restrict__ groups, int n_groups, float4* __restrict__ acc,
+                 uint32_t* __restrict__ queue, uint32_t* __restrict__ status, int2* __restrict__ gstack,
+                 int gstack_cap, WalkEpilogue ep, WalkFrontier fr) {
+    using Smem = PairSmem<H>;
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    const int id = threadIdx.x >> 6;         // pair of the block
+    const int w = (threadIdx.x >> 5) & 1;    // which of its two warps
+    Smem& W = reinterpret_cast<Smem*>(walk_smem)[id];
+    int2* const gstk = gstack + ((size_t)blockIdx.x * kPairBlockPairs + id) * (size_t)gstack_cap;
+    const int lane = threadIdx.x & 31;
+    const uint32_t lane_bit = 1u << lane;
+    const uint32_t lt = lane_bit - 1u;
+    const float G = wp.G, eps2 = wp.eps2, theta2 = wp.theta2;
+    const float2 e2 = make_float2(eps2, eps2), th2 = make_float2(theta2, theta2);
+    const float leaf_thr = __fmul_rn(eps2, 1.01f);
+    const float k_take = theta2 * kBoxLo, k_open = theta2 * kBoxHi;
+    const int batch = wp.batch;
+    const float4 empty = make_float4(1e30f, 1e30f, 1e30f, 0.0f);
+
+    for (;;) {
+        if (w == 0 && lane == 0) W.item = (int)atomicAdd(queue, 1u);
+        pair_sync(id);
+        const int g = W.item;
+        if (g >= n_groups) break;
+        const WalkGroup grp = groups[g];
+        const bool valid = lane < grp.count;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (valid) {
+            const int j = grp.start + lane;
+            p = __ldg(pos + (fr.perm ? __ldg(fr.perm + j) : j));
+        }
+        const uint32_t live = __ballot_sync(kFull, valid);
+        Targets<1> X;
+        X.npx[0] = make_float2(-p.x, -p.x);
+        X.npy[0] = make_float2(-p.y, -p.y);
+        X.npz[0] = make_float2(-p.z, -p.z);
+        float3 box_lo = make_float3(INFINITY, INFINITY, INFINITY);
+        float3 box_hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
+        if (valid) {
+            box_lo = make_float3(fminf(box_lo.x, p.x), fminf(box_lo.y, p.y), fminf(box_lo.z, p.z));
+            box_hi = make_float3(fmaxf(box_hi.x, p.x), fmaxf(box_hi.y, p.y), fmaxf(box_hi.z, p.z));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            box_lo.x = fminf(box_lo.x, __shfl_xor_sync(kFull, box_lo.x, o));
+            box_lo.y = fminf(box_lo.y, __shfl_xor_sync(kFull, box_lo.y, o));
+            box_lo.z = fminf(box_lo.z, __shfl_xor_sync(kFull, box_lo.z, o));
+            box_hi.x = fmaxf(box_hi.x, __shfl_xor_sync(kFull, box_hi.x, o));
+            box_hi.y = fmaxf(box_hi.y, __shfl_xor_sync(kFull, box_hi.y, o));
+            box_hi.z = fmaxf(box_hi.z, __shfl_xor_sync(kFull, box_hi.z, o));
+        }
+        Half2Sums A = {0.f, 0.f, 0.f, 0.f};
+        const int s = grp.seg;
+        const int off = (int)__ldg(L.seg_off + s);
+        const int seg_n = (int)__ldg(L.seg_off + s + 1) - off;
+        int nsrc = 0;
+        const auto& mine = W.half[w];  // the lists of this warp's parity
+
+        if (seg_n >= 2) {
+            int top = 0, gtop = 0;
+            int4 fm = make_int4(0, 0, 0, 0);
+            if (fr.meta) fm = fr.meta[grp.super];
+            if (fm.w && fm.z - Smem::kSpillAbove <= gstack_cap) {
+                const int32_t* tl = fr.list + (size_t)grp.super * kSuperCap;
+                for (int base = 0; base < fm.x; base += kSrcCap) {
+                    const int cnt = min(kSrcCap, fm.x - base);
+                    const int slots = (cnt + 3) & ~3;
+                    pair_sync(id);
+                    for (int e = lane + 32 * w; e < slots; e += 64) {
+                        float4 q = empty;
+                        if (e < cnt) q = __ldg(&wn[__ldg(tl + base + e)].cm);
+                        put_entry(W.half[e & 1].sxy, W.half[e & 1].szm, e >> 1, q);
+                    }
+                    pair_sync(id);
+#pragma unroll 4
+                    for (int q = 0; q < (slots >> 2); ++q) {
+                        const float4 zm = mine.szm[q];
+                        const PairD d = pair_d_take(mine.sxy[q], zm, X.npx[0], X.npy[0], X.npz[0], e2);
+                        half_add<kPot>(A, d, zm, true, true);
+                    }
+                }
+                const int32_t* sl = fr.src + (size_t)grp.super * kSuperSrcCap;
+                for (int base = 0; base < fm.y; base += kSrcCap) {
+                    const int cnt = min(kSrcCap, fm.y - base);
+                    for (int e = lane + 32 * w; e < cnt; e += 64) {
+                        W.srcp[e] = __ldg(sl + base + e);
+                        W.srcm[e] = live;
+                    }
+                    flush_pair<H, kPot>(W, cnt, id, w, lane, lane_bit, pos, G, X, e2, leaf_thr, A);
+                }
+                const int32_t* fl = tl + kSuperCap - fm.z;
+                const int to_g = max(0, fm.z - Smem::kSpillAbove);
+                const int at = lane + 32 * w;
+                for (int j = at; j < to_g; j += 64) gstk[j] = make_int2(__ldg(fl + j), (int)live);
+                for (int j = at; j < fm.z - to_g; j += 64) W.stk[j] = make_int2(__ldg(fl + to_g + j), (int)live);
+                gtop = to_g;
+                top = fm.z - to_g;
+            } else {
+                if (w == 0 && lane == 0) W.stk[0] = make_int2(off - s, (int)live);
+                top = 1;
+            }
+            if (gtop > 0) __threadfence_block();
+            pair_sync(id);
+            int pop_budget = seg_n - 1;
+            while (top > 0 || gtop > 0) {
+                // refill the shared top from the global bottom when it runs low
+                if (top < batch && gtop > 0) {
+                    const int k = gtop < kSpillCount ? gtop : kSpillCount;
+                    if (w == 0) {
+                        int2 keep[H];
+#pragma unroll
+                        for (int h = 0; h < H; ++h) keep[h] = lane + 32 * h < top ? W.stk[lane + 32 * h] : int2{};
+                        __syncwarp();
+#pragma unroll
+                        for (int h = 0; h < H; ++h)
+                            if (lane + 32 * h < top) W.stk[k + lane + 32 * h] = keep[h];
+                        for (int j = lane; j < k; j += 32) W.stk[j] = __ldcg(gstk + gtop - k + j);
+                    }
+                    gtop -= k;
+                    top += k;
+                    pair_sync(id);
+                }
+                const int b = top < batch ? top : batch;
+                pop_budget -= b;
+                if (pop_budget < 0) {
+                    if (w == 0 && lane == 0) atomicOr(status, GCS_DEV_TREE_MALFORMED);
+                    break;
+                }
+                top -= b;
+                // 1-2. fetch and classify node lane + 32 w
+                int code_a = 0, code_b = kWalkSkipTag, cls = kClassNone;
+                uint32_t my_mask = 0u;
+                float4 com = make_float4(0.f, 0.f, 0.f, 0.f);
+                float w2 = 0.0f;
+                if (lane + 32 * w < b) {
+                    const int2 e = W.stk[top + lane + 32 * w];
+                    const float4* np = reinterpret_cast<const float4*>(wn + e.x);
+                    com = __ldg(np);
+                    const int4 k = __ldg(reinterpret_cast<const int4*>(np + 1));
+                    w2 = __int_as_float(k.x);
+                    code_a = k.y;
+                    code_b = k.z;
+                    my_mask = (uint32_t)e.y;
+                    cls = box_class(com, w2, box_lo, box_hi, eps2, k_take, k_open);
+                    if (cls == kClassTake && my_mask == live) cls = kClassTakeFull;
+                }
+                // compact into three lists, the other warp's nodes after
+                // (w = 0) or before (w = 1) this one's
+                const uint32_t bf = __ballot_sync(kFull, cls == kClassTakeFull);
+                const uint32_t bt = __ballot_sync(kFull, cls == kClassTake);
+                const uint32_t bm = __ballot_sync(kFull, cls == kClassMixed);
+                if (lane == 0) {
+                    W.ball[w][0] = bf;
+                    W.ball[w][1] = bt;
+                    W.ball[w][2] = bm;
+                }
+                pair_sync(id);
+                const int of = __popc(W.ball[w ^ 1][0]), ot = __popc(W.ball[w ^ 1][1]), om = __popc(W.ball[w ^ 1][2]);
+                const int n_full = __popc(bf) + of, n_take = __popc(bt) + ot, n_mixed = __popc(bm) + om;
+                // first pair of each list
+                const int take_at = (n_full + 3) >> 2;
+                const int mixed_at = take_at + ((n_take + 3) >> 2);
+                const int lists_end = mixed_at + ((n_mixed + 3) >> 2);
+                const int rank = cls == kClassTakeFull ? __popc(bf & lt) + (w ? of : 0)
+                               : cls == kClassTake ? 4 * take_at + __popc(bt & lt) + (w ? ot : 0)
+                               : cls == kClassMixed ? 4 * mixed_at + __popc(bm & lt) + (w ? om : 0) : -1;
+                if (rank >= 0) {
+                    auto& S = W.half[rank & 1];
+                    put_entry(S.xy, S.zm, rank >> 1, com);
+                    put_mask(S.mask, rank >> 1, my_mask);
+                    reinterpret_cast<float*>(S.w2 + (rank >> 2))[(rank >> 1) & 1] = w2;
+                }
+                if (w == 0) {  // empty entries to whole pairs: up to three a list
+                    const int list = lane / 3, k = lane - 3 * list;
+                    const int at = list == 0 ? n_full + k : list == 1 ? 4 * take_at + n_take + k
+                                                                      : 4 * mixed_at + n_mixed + k;
+                    const int end = list == 0 ? 4 * take_at : list == 1 ? 4 * mixed_at : 4 * lists_end;
+                    if (lane < 9 && at < end) {
+                        auto& S = W.half[at & 1];
+                        put_entry(S.xy, S.zm, at >> 1, empty);
+                        put_mask(S.mask, at >> 1, 0u);
+                        reinterpret_cast<float*>(S.w2 + (at >> 2))[(at >> 1) & 1] = 0.0f;
+                    }
+                }
+                pair_sync(id);
+                // 3a. nodes every live target accepts
+#pragma unroll 4
+                for (int q = 0; q < take_at; ++q) {
+                    const float4 zm = mine.zm[q];
+                    const PairD d = pair_d_take(mine.xy[q], zm, X.npx[0], X.npy[0], X.npz[0], e2);
+                    half_add<kPot>(A, d, zm, true, true);
+                }
+                // 3b. nodes accepted by every target of their masks
+#pragma unroll 4
+                for (int q = take_at; q < mixed_at; ++q) {
+                    const float4 zm = mine.zm[q];
+                    const uint2 mk = mine.mask[q];
+                    const PairD d = pair_d_take(mine.xy[q], zm, X.npx[0], X.npy[0], X.npz[0], e2);
+                    half_add<kPot>(A, d, zm, (mk.x & lane_bit) != 0u, (mk.y & lane_bit) != 0u);
+                }
+                // 3c. mixed nodes: each target's own test
+#pragma unroll 2
+                for (int q = mixed_at; q < lists_end; ++q) {
+                    const float4 zm = mine.zm[q];
+                    const float2 w2q = mine.w2[q];
+                    const uint2 mk = mine.mask[q];
+                    const PairD d = pair_d(mine.xy[q], zm, X.npx[0], X.npy[0], X.npz[0], e2);
+                    const float2 lim = __fmul2_rn(d.d2, th2);  // accept_monopole: w^2 < d2 * theta^2
+                    const bool act0 = (mk.x & lane_bit) != 0u, act1 = (mk.y & lane_bit) != 0u;
+                    const bool take0 = w2q.x < lim.x, take1 = w2q.y < lim.y;
+                    half_add<kPot>(A, d, zm, act0 && take0, act1 && take1);
+                    const uint32_t om0 = __ballot_sync(kFull, act0 && !take0);
+                    const uint32_t om1 = __ballot_sync(kFull, act1 && !take1);
+                    if (lane == 0) W.half[w].nopen[q] = make_uint2(om0, om1);
+                }
+                pair_sync(id);
+                // 4. parallel push / append for the opened nodes, in the order
+                // of the one-warp kernel: by lane, its two nodes one after the
+                // other
+                const uint32_t my_open =
+                    cls == kClassOpen ? my_mask
+                    : cls == kClassMixed
+                        ? reinterpret_cast<const uint32_t*>(&W.half[rank & 1].nopen[rank >> 2])[(rank >> 1) & 1] : 0u;
+                int n_push = 0, n_src = 0;
+                if (my_open != 0u && code_b != kWalkSkipTag) {
+                    if (code_b >= kWalkBucketTag) {
+                        n_src = code_b - kWalkBucketTag;
+                    } else {
+                        n_push = (code_a >= 0) + (code_b >= 0);
+                        n_src = (code_a < 0) + (code_b < 0);
+                    }
+                }
+                const uint32_t own = ((uint32_t)n_push << 16) | (uint32_t)n_src;
+                W.cnt[w][lane] = own;
+                pair_sync(id);
+                const uint32_t other = W.cnt[w ^ 1][lane];
+                const uint32_t excl = warp_exclusive_scan(own + other, lane);
+                const uint32_t total = __shfl_sync(kFull, excl + own + other, 31);
+                const uint32_t first = excl + (w ? other : 0u);  // this node's pushes and sources
+                if (n_push > 0) {
+                    int at = top + (int)(first >> 16);
+                    if (code_a >= 0) W.stk[at++] = make_int2(code_a, (int)my_open);
+                    if (code_b >= 0) W.stk[at++] = make_int2(code_b, (int)my_open);
+                }
+                top += (int)(total >> 16);
+                const int add = (int)(total & 0xFFFFu);
+                if (add > 0) {
+                    // one descriptor per node with sources, in source order
+                    const bool other_src = (other & 0xFFFFu) != 0u;
+                    const uint32_t bs = __ballot_sync(kFull, n_src > 0), bo = __ballot_sync(kFull, other_src);
+                    const int n_desc = __popc(bs) + __popc(bo);
+                    if (n_src > 0) {
+                        const int d = __popc(bs & lt) + __popc(bo & lt) + (w && other_src ? 1 : 0);
+                        W.sdesc[d] = make_int4((int)(first & 0xFFFFu), code_a, code_b, 0);
+                        W.dmask[d] = my_open;
+                    }
+                    pair_sync(id);
+                    for (int base = 0; base < add;) {
+                        if (nsrc == kSrcCap) {
+                            flush_pair<H, kPot>(W, nsrc, id, w, lane, lane_bit, pos, G, X, e2, leaf_thr, A);
+                            nsrc = 0;
+                        }
+                        const int window = min(kSrcCap - nsrc, add - base);
+                        for (int j = base + lane + 32 * w; j < base + window; j += 64) {
+                            // the last descriptor starting at or before j
+                            int lo = 0, hi = n_desc - 1;
+                            while (lo < hi) {
+                                const int mid = (lo + hi + 1) >> 1;
+                                if (W.sdesc[mid].x <= j) lo = mid;
+                                else hi = mid - 1;
+                            }
+                            const int4 e = W.sdesc[lo];
+                            const int r = j - e.x;  // r-th source of that node
+                            const int at = nsrc + (j - base);
+                            W.srcp[at] = e.z >= kWalkBucketTag ? e.y + r : ((r == 0 && e.y < 0) ? ~e.y : ~e.z);
+                            W.srcm[at] = W.dmask[lo];
+                        }
+                        nsrc += window;
+                        base += window;
+                    }
+                }
+                pair_sync(id);
+                if (nsrc >= 32) {
+                    flush_pair<H, kPot>(W, nsrc, id, w, lane, lane_bit, pos, G, X, e2, leaf_thr, A);
+                    nsrc = 0;
+                }
+                // spill the shared stack's bottom before it can overflow
+                if (top > Smem::kSpillAbove) {
+                    const int rest = top - kSpillCount;
+                    const bool fits = gtop + kSpillCount <= gstack_cap;
+                    if (w == 0) {
+                        if (fits) {
+                            for (int j = lane; j < kSpillCount; j += 32) gstk[gtop + j] = W.stk[j];
+                        } else if (lane == 0) {
+                            atomicOr(status, GCS_DEV_WALK_STACK_OVERFLOW);
+                        }
+                        constexpr int kMove = (Smem::kStackCap - kSpillCount + 31) / 32;
+                        int2 mv[kMove];
+#pragma unroll
+                        for (int i = 0; i < kMove; ++i) {
+                            const int j = lane + 32 * i;
+                            mv[i] = j < rest ? W.stk[kSpillCount + j] : int2{};
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < kMove; ++i) {
+                            const int j = lane + 32 * i;
+                            if (j < rest) W.stk[j] = mv[i];
+                        }
+                    }
+                    if (fits) gtop += kSpillCount;
+                    top = rest;
+                    pair_sync(id);
+                }
+            }
+        }
+        if (nsrc > 0) flush_pair<H, kPot>(W, nsrc, id, w, lane, lane_bit, pos, G, X, e2, leaf_thr, A);
+        if (w == 1) W.sums[lane] = make_float4(A.ax, A.ay, A.az, A.pot);
+        pair_sync(id);
+        if (w == 1) continue;
+        if (valid) {
+            const int j = grp.start + lane;
+            const int64_t i = fr.perm ? __ldg(fr.perm + j) : j;  // the target's particle
+            const float4 o = W.sums[lane];
+            const float4 a = make_float4(__fadd_rn(A.ax, o.x), __fadd_rn(A.ay, o.y), __fadd_rn(A.az, o.z),
+                                         __fadd_rn(A.pot, o.w));
+            finish_target(pos, acc, ep, i, a);
+        }
+        if (ep.vel_in && ep.host_flags) {
+            __syncwarp();
+            if (lane == 0) finish_group(ep, g);
+        }
+        __syncwarp();
+    }
+    // (as in walk_kernel, with a count per pair)
+    if (w == 0 && lane == 0) {
+        const uint32_t total = gridDim.x * kPairBlockPairs;
         if (atomicAdd(queue + 1, 1u) == total - 1) {
             queue[0] = 0u;
             queue[1] = 0u;
@@ -1139,6 +1603,15 @@ int occupancy_of() {
     return nb > 0 ? nb : 1;
 }
 
+template <int H, bool kPot>
+void configure_pair() {
+    static std::once_flag done[kMaxDevices];
+    once_per_device(done, [] {
+        cudaFuncSetAttribute(walk_pair_kernel<H, kPot>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(PairSmem<H>) * kPairBlockPairs));
+    });
+}
+
 template <int T>
 int max_blocks_of(int batch, int with_potential) {
     // per device (the query needs the device's attribute opt-in first)
@@ -1207,6 +1680,33 @@ static void launch_ht(const Layout& L, const WalkParams& q, const float4* pos, c
     }
 }
 
+// Whether every group gets two warps: while all groups find a pair of warps
+// within two waves.  Walk stage in us, one warp a group / two (theta 0.5, leaf
+// 8, batch 64 from 16,384 on):
+//    1,408 particles  78 /  61       60,000 (0.7, leaf 4)     170 / 139
+//    8,192           170 / 121       75,000                   326 / 285
+//   16,384           199 / 135       110,000                  406 / 385
+//   45,056           309 / 225       131,072 (0.7, leaf 4)    289 / 295
+//   16 x 5,000       170 / 152       262,144                  737 / 770
+static bool pairs_pay(int n_groups, int sm_count) { return n_groups <= 20 * sm_count; }
+
+template <int H>
+static void launch_pairs(const Layout& L, const WalkParams& q, const float4* pos, const WalkNode* wn,
+                         const WalkGroup* groups, int n_groups, float4* acc, uint32_t* queue, uint32_t* status,
+                         int2* gstack, int cap, unsigned g, cudaStream_t st, const WalkEpilogue& ep,
+                         const WalkFrontier& fr) {
+    const size_t sm = sizeof(PairSmem<H>) * kPairBlockPairs;
+    if (q.with_potential) {
+        configure_pair<H, true>();
+        walk_pair_kernel<H, true><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue, status,
+                                                               gstack, cap, ep, fr);
+    } else {
+        configure_pair<H, false>();
+        walk_pair_kernel<H, false><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue, status,
+                                                                gstack, cap, ep, fr);
+    }
+}
+
 void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
                  const WalkNode* wn, const WalkGroup* groups, int n_groups, int targets_per_lane, float4* acc,
                  uint32_t* queue, uint32_t* status, int blocks_per_sm, int sm_count,
@@ -1259,6 +1759,19 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
     // entries per warp region: the whole buffer split over this grid's warps
     const size_t units = gstack_entries / ((size_t)grid * kWalkWarps);
     const int cap = (int)(std::min<size_t>(units, (size_t)1 << 24) / (size_t)T);
+    if (T == 1 && !counts && pairs_pay(n_groups, sm_count)) {
+        // two warps a group; the stack regions are shared out over the pairs
+        const int64_t blocks = ((int64_t)n_groups + kPairBlockPairs - 1) / kPairBlockPairs;
+        const int64_t pairs = blocks * kPairBlockPairs;
+        const int pair_cap = (int)std::min<size_t>(gstack_entries / (size_t)pairs, (size_t)1 << 24);
+        if (q.batch > 32)
+            launch_pairs<2>(L, q, pos, wn, groups, n_groups, acc, queue, status, gstack, pair_cap, (unsigned)blocks, st,
+                            ep, fr);
+        else
+            launch_pairs<1>(L, q, pos, wn, groups, n_groups, acc, queue, status, gstack, pair_cap, (unsigned)blocks, st,
+                            ep, fr);
+        return;
+    }
     if (T == 2) {
         if (q.batch > 32)
             launch_ht<2, 2>(L, q, pos, wn, groups, n_groups, acc, queue, status, counts, gstack, cap, g, st, ep, fr);
