@@ -21,6 +21,7 @@
 
 #include "gcs_internal.h"
 #include "device_math.cuh"
+#include "pdl.cuh"
 
 namespace gcs {
 
@@ -77,6 +78,9 @@ front_kernel(const float4* __restrict__ pos, int n, int front_bounds, float gmin
     const int tile_base = rank * kTile;
     const int warp_at = warp * (kItems * 32);  // the warp's first pair in the tile
     const uint32_t lt_mask = (1u << lane) - 1u;
+
+    let_next_start();
+    wait_for_previous();
 
     // ---- particles, bounds, keys
     float4 p[kItems];
@@ -257,18 +261,20 @@ void configure_front() {
 }
 
 template <int kItems>
-cudaLaunchConfig_t front_config(int blocks, cudaLaunchAttribute* attr, cudaStream_t st) {
+cudaLaunchConfig_t front_config(int blocks, cudaLaunchAttribute (&attr)[2], cudaStream_t st) {
     configure_front<kItems>();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(kFrontThreads);
     cfg.dynamicSmemBytes = sizeof(FrontSmem<kItems>);
     cfg.stream = st;
-    attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = (unsigned)blocks;
-    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (pdl.cuh)
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cfg;
 }
 
@@ -308,8 +314,8 @@ bool front_available() {
     for (int items : {1, 2, 3, 4, 6})
         with_items(items, [&](auto k) {
             constexpr int kItems = decltype(k)::value;
-            cudaLaunchAttribute attr;
-            const cudaLaunchConfig_t cfg = front_config<kItems>(16, &attr, nullptr);
+            cudaLaunchAttribute attr[2];
+            const cudaLaunchConfig_t cfg = front_config<kItems>(16, attr, nullptr);
             int clusters = 0;
             if (cudaOccupancyMaxActiveClusters(&clusters, front_kernel<kItems>, &cfg) != cudaSuccess || clusters < 1)
                 ok = false;
@@ -324,8 +330,8 @@ void launch_front(const float4* pos, int n, int front_bounds, float gmin, float 
     const FrontShape shape = front_shape(n);
     with_items(shape.items, [&](auto k) {
         constexpr int kItems = decltype(k)::value;
-        cudaLaunchAttribute attr;
-        const cudaLaunchConfig_t cfg = front_config<kItems>(shape.blocks, &attr, st);
+        cudaLaunchAttribute attr[2];
+        const cudaLaunchConfig_t cfg = front_config<kItems>(shape.blocks, attr, st);
         cudaLaunchKernelEx(&cfg, front_kernel<kItems>, pos, n, front_bounds, gmin, gmax, seg_bounds, keys, idx, status);
     });
 }

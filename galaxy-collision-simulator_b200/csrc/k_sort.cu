@@ -48,6 +48,7 @@
 #include <type_traits>
 
 #include "gcs_internal.h"
+#include "pdl.cuh"
 
 namespace gcs {
 
@@ -130,11 +131,13 @@ onesweep_kernel(Layout L, int shift, const uint64_t* __restrict__ keys_in,
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int n = L.n;
 
+    let_next_start();
+    for (int i = t; i < kWarps * kRadix; i += kThreads) (&S.whist[0][0])[i] = 0;
+    wait_for_previous();
     if (t == 0) {
         S.tile = atomicAdd(tile_counter, 1u);
         S.bad = 0;
     }
-    for (int i = t; i < kWarps * kRadix; i += kThreads) (&S.whist[0][0])[i] = 0;
     const uint32_t h = t < kRadix ? hist[t] : 0u;  // t == digit
     __syncthreads();
     const int tile = (int)S.tile;
@@ -282,12 +285,13 @@ void launch_tiles(const Layout& L, int pass, int tiles, const uint64_t* keys_in,
                              (int)smem_seg);
     });
     if (pass < kKeyPasses) {
-        onesweep_kernel<kThreads, kItems, false><<<(unsigned)tiles, kThreads, smem_key, st>>>(
-            L, kRadixBits * pass, keys_in, vals_in, keys_out, vals_out, hist, tile_counter, lookback, status, tiles);
+        launch_after(onesweep_kernel<kThreads, kItems, false>, (unsigned)tiles, kThreads, smem_key, st, L,
+                     kRadixBits * pass, keys_in, vals_in, keys_out, vals_out, hist, tile_counter, lookback, status,
+                     tiles);
     } else {
-        onesweep_kernel<kThreads, kItems, true><<<(unsigned)tiles, kThreads, smem_seg, st>>>(
-            L, kRadixBits * (pass - kKeyPasses), keys_in, vals_in, keys_out, vals_out, hist, tile_counter, lookback,
-            status, tiles);
+        launch_after(onesweep_kernel<kThreads, kItems, true>, (unsigned)tiles, kThreads, smem_seg, st, L,
+                     kRadixBits * (pass - kKeyPasses), keys_in, vals_in, keys_out, vals_out, hist, tile_counter,
+                     lookback, status, tiles);
     }
 }
 

@@ -9,6 +9,7 @@
 
 #include "gcs_internal.h"
 #include "device_math.cuh"
+#include "pdl.cuh"
 
 namespace gcs {
 
@@ -102,6 +103,8 @@ __global__ void pack_playback_kernel(const float4* __restrict__ pos, const float
 __global__ void bounds_kernel(const float4* __restrict__ pos, const Chunk* __restrict__ chunks,
                               int n_chunks, uint32_t* __restrict__ bounds_enc,
                               uint32_t* __restrict__ status) {
+    let_next_start();
+    wait_for_previous();
     constexpr int kInFlight = 8;  // independent loads per thread per sweep
     __shared__ float s_lo[kStreamThreads / 32], s_hi[kStreamThreads / 32];
     for (int c = blockIdx.x; c < n_chunks; c += gridDim.x) {
@@ -150,6 +153,8 @@ __global__ void bounds_kernel(const float4* __restrict__ pos, const Chunk* __res
 
 __global__ void bounds_decode_kernel(const uint32_t* __restrict__ enc, float2* __restrict__ out,
                                      int nseg) {
+    let_next_start();
+    wait_for_previous();
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x)
         out[s] = make_float2(ordered_to_float(~enc[2 * s]), ordered_to_float(enc[2 * s + 1]));
 }
@@ -165,8 +170,10 @@ __global__ void encode_kernel(Layout L, const float4* __restrict__ pos, int boun
                               uint32_t* __restrict__ hist, int n_seg_passes) {
     __shared__ uint32_t s_hist[kMaxPasses][kRadix];
     const int passes = kKeyPasses + n_seg_passes;
+    let_next_start();
     for (int t = threadIdx.x; t < passes * kRadix; t += blockDim.x) (&s_hist[0][0])[t] = 0;
     __syncthreads();
+    wait_for_previous();
     float lo = gmin, scale = 0.0f;
     int cur_seg = -1;
     if (bounds_mode == GCS_BOUNDS_CALLER) scale = morton_scale(gmin, gmax);
@@ -416,20 +423,19 @@ void launch_bounds(const Layout& L, const float4* pos, const Chunk* chunks, int 
     if (n_chunks <= 0) return;
     int grid = stream_grid(L.n);
     if (grid > n_chunks) grid = n_chunks;
-    bounds_kernel<<<grid, kStreamThreads, 0, st>>>(pos, chunks, n_chunks, bounds_enc, status);
+    launch_after(bounds_kernel, grid, kStreamThreads, 0, st, pos, chunks, n_chunks, bounds_enc, status);
 }
 
 void launch_bounds_decode(const uint32_t* bounds_enc, float2* bounds, int nseg, cudaStream_t st) {
-    bounds_decode_kernel<<<(nseg + 255) / 256, 256, 0, st>>>(bounds_enc, bounds, nseg);
+    launch_after(bounds_decode_kernel, (nseg + 255) / 256, 256, 0, st, bounds_enc, bounds, nseg);
 }
 
 void launch_encode(const Layout& L, const float4* pos, int bounds_mode, float gmin, float gmax,
                    const float2* seg_bounds, uint64_t* keys, uint32_t* idx, uint32_t* hist,
                    int n_seg_passes, cudaStream_t st) {
     if (L.n <= 0) return;
-    encode_kernel<<<stream_grid(L.n), kStreamThreads, 0, st>>>(L, pos, bounds_mode, gmin, gmax,
-                                                                seg_bounds, keys, idx, hist,
-                                                                n_seg_passes);
+    launch_after(encode_kernel, stream_grid(L.n), kStreamThreads, 0, st, L, pos, bounds_mode, gmin, gmax, seg_bounds,
+                 keys, idx, hist, n_seg_passes);
 }
 
 void launch_gather(const uint32_t* idx, const float4* pos_in, const float4* vel_in, float4* pos_out,

@@ -23,6 +23,7 @@
 // the tree), rounded once to FP32.
 #include "gcs_internal.h"
 #include "device_math.cuh"
+#include "pdl.cuh"
 
 namespace gcs {
 
@@ -107,6 +108,8 @@ __global__ void build_kernel(Layout L, const uint64_t* __restrict__ keys,
                              int32_t* __restrict__ leaf_parent, WalkNode* __restrict__ wn,
                              double4* __restrict__ com64, uint32_t* __restrict__ agg_ticket,
                              uint32_t* __restrict__ status) {
+    let_next_start();
+    wait_for_previous();
     if (blockIdx.x == 0 && threadIdx.x == 0) *agg_ticket = 0u;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < L.n; g += gridDim.x * blockDim.x) {
         const int s = L.nseg > 1 ? __ldg(L.seg_id + g) : 0;
@@ -213,6 +216,8 @@ __device__ __forceinline__ void write_walk_node(const WalkNodeParams& wnp, int n
 // internal node g - s exists for every particle but the last of segment s.
 __global__ void walk_nodes_kernel(Layout L, const BvhNodeTraverse* __restrict__ tr, WalkNodeParams wnp,
                                   uint32_t* __restrict__ status) {
+    let_next_start();
+    wait_for_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= L.n) return;
     const int s = L.nseg > 1 ? __ldg(L.seg_id + g) : 0;
@@ -312,6 +317,7 @@ aggregate_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __re
     }
     const int b0 = blockIdx.x * kAggRange;
     const int count = min(kAggRange, L.n - b0);
+    let_next_start();
     const auto seg_of = [&](int g) { return L.nseg > 1 ? (int)__ldg(L.seg_id + g) : 0; };
     const auto seg_end = [&](int s) { return L.nseg > 1 ? (int)__ldg(L.seg_off + s + 1) : L.n; };
 
@@ -498,6 +504,8 @@ rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restric
             const uint32_t* __restrict__ n_roots, int n_runs, int com_fp64, WalkNodeParams wnp,
             uint32_t* __restrict__ ticket, uint32_t* __restrict__ status) {
     __shared__ int s_block;
+    let_next_start();
+    wait_for_previous();
     if (threadIdx.x == 0) s_block = (int)atomicAdd(ticket, 1u);
     __syncthreads();
     const int run = s_block * kRiseWarps + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -605,6 +613,8 @@ rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restric
 // walk_nodes_kernel).
 __global__ void relay_reset_kernel(Layout L, BvhNodeTraverse* __restrict__ tr, WalkNode* __restrict__ wn,
                                    double4* __restrict__ com64, uint32_t* __restrict__ ticket) {
+    let_next_start();
+    wait_for_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g == 0) *ticket = 0u;
     if (g >= L.n) return;
@@ -625,13 +635,13 @@ void launch_build(const Layout& L, const uint64_t* keys, BvhNodeTraverse* tr, Bv
                   int32_t* leaf_parent, WalkNode* wn, double4* com64, uint32_t* agg_ticket, uint32_t* status,
                   cudaStream_t st) {
     if (L.n <= 0) return;
-    build_kernel<<<tree_grid(L.n), 256, 0, st>>>(L, keys, tr, bd, leaf_parent, wn, com64, agg_ticket, status);
+    launch_after(build_kernel, tree_grid(L.n), 256, 0, st, L, keys, tr, bd, leaf_parent, wn, com64, agg_ticket, status);
 }
 
 void launch_relay_reset(const Layout& L, BvhNodeTraverse* tr, WalkNode* wn, double4* com64, uint32_t* agg_ticket,
                         cudaStream_t st) {
     if (L.n <= 0) return;
-    relay_reset_kernel<<<tree_grid(L.n), 256, 0, st>>>(L, tr, wn, com64, agg_ticket);
+    launch_after(relay_reset_kernel, tree_grid(L.n), 256, 0, st, L, tr, wn, com64, agg_ticket);
 }
 
 void launch_aggregate(const Layout& L, const float4* pos, BvhNodeTraverse* tr, BvhNodeBuild* bd,
@@ -639,16 +649,18 @@ void launch_aggregate(const Layout& L, const float4* pos, BvhNodeTraverse* tr, B
                       int2* roots, uint32_t* n_roots, uint32_t* agg_ticket, uint32_t* status, cudaStream_t st) {
     if (L.n <= 0) return;
     const int runs = (L.n + kAggRange - 1) / kAggRange;
+    // (launched plainly: early blocks would hold shared memory that the gather
+    // beside the build needs; 344 against 351 us a step of 45,056 particles)
     aggregate_kernel<<<(unsigned)runs, kAggThreads, 0, st>>>(L, pos, tr, bd, leaf_parent, wnp, roots, n_roots, status);
     if (runs > 1)  // one block's nodes are all local
-        rise_kernel<<<(unsigned)((runs + kRiseWarps - 1) / kRiseWarps), kRiseWarps * 32, 0, st>>>(
-            L, pos, tr, bd, com64, leaf_parent, roots, n_roots, runs, com_fp64, wnp, agg_ticket, status);
+        launch_after(rise_kernel, (unsigned)((runs + kRiseWarps - 1) / kRiseWarps), kRiseWarps * 32, 0, st, L, pos, tr,
+                     bd, com64, leaf_parent, roots, n_roots, runs, com_fp64, wnp, agg_ticket, status);
 }
 
 void launch_walk_nodes(const Layout& L, const BvhNodeTraverse* tr, WalkNodeParams wnp, uint32_t* status,
                        cudaStream_t st) {
     if (L.n <= 0 || !wnp.wn) return;
-    walk_nodes_kernel<<<tree_grid(L.n), 256, 0, st>>>(L, tr, wnp, status);
+    launch_after(walk_nodes_kernel, tree_grid(L.n), 256, 0, st, L, tr, wnp, status);
 }
 
 }  // namespace gcs

@@ -69,6 +69,7 @@
 
 #include "gcs_internal.h"
 #include "device_math.cuh"
+#include "pdl.cuh"
 
 namespace gcs {
 
@@ -1348,6 +1349,8 @@ __global__ void __launch_bounds__(kPartWarps * 32)
 partition_kernel(const float4* __restrict__ pos, const SuperGroup* __restrict__ supers, int n_supers, int levels,
                  int32_t* __restrict__ perm) {
     __shared__ float sp[kPartWarps][3][kSuperTargets];
+    let_next_start();
+    wait_for_previous();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sgi = blockIdx.x * kPartWarps + warp;
     if (sgi >= n_supers) return;
@@ -1453,6 +1456,8 @@ __global__ void __launch_bounds__(kFrontWarps * 32)
 frontier_kernel(Layout L, const float4* __restrict__ pos, const WalkNode* __restrict__ wn, WalkFrontier fr,
                 float eps2, float theta2, uint32_t* __restrict__ status) {
     __shared__ int32_t stk_all[kFrontWarps][kFrontStack];
+    let_next_start();
+    wait_for_previous();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sgi = blockIdx.x * kFrontWarps + warp;
     if (sgi >= fr.n_supers) return;
@@ -1662,21 +1667,21 @@ static void launch_ht(const Layout& L, const WalkParams& q, const float4* pos, c
     if (counts) {
         if (q.with_potential) {
             configure<H, T, true, true>();
-            walk_kernel<H, T, true, true><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue,
-                                                                       status, counts, gs, cap, ep, fr);
+            walk_kernel<H, T, true, true><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue, status,
+                                                               counts, gs, cap, ep, fr);
         } else {
             configure<H, T, false, true>();
-            walk_kernel<H, T, false, true><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue,
-                                                                        status, counts, gs, cap, ep, fr);
+            walk_kernel<H, T, false, true><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue, status,
+                                                               counts, gs, cap, ep, fr);
         }
     } else if (q.with_potential) {
         configure<H, T, true, false>();
-        walk_kernel<H, T, true, false><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue,
-                                                                    status, nullptr, gs, cap, ep, fr);
+        walk_kernel<H, T, true, false><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue, status,
+                                                               nullptr, gs, cap, ep, fr);
     } else {
         configure<H, T, false, false>();
-        walk_kernel<H, T, false, false><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue,
-                                                                     status, nullptr, gs, cap, ep, fr);
+        walk_kernel<H, T, false, false><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue, status,
+                                                               nullptr, gs, cap, ep, fr);
     }
 }
 
@@ -1703,7 +1708,7 @@ static void launch_pairs(const Layout& L, const WalkParams& q, const float4* pos
     } else {
         configure_pair<H, false>();
         walk_pair_kernel<H, false><<<g, kWalkThreads, sm, st>>>(L, q, pos, wn, groups, n_groups, acc, queue, status,
-                                                                gstack, cap, ep, fr);
+                                                               gstack, cap, ep, fr);
     }
 }
 
@@ -1732,7 +1737,7 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
         } else {
             fr.perm = nullptr;
         }
-        frontier_kernel<<<fb, kFrontWarps * 32, 0, st>>>(L, pos, wn, fr, wp.eps2, wp.theta2, status);
+        launch_after(frontier_kernel, fb, kFrontWarps * 32, 0, st, L, pos, wn, fr, wp.eps2, wp.theta2, status);
         if (joined) cudaStreamWaitEvent(st, fr.join, 0);
     } else {
         fr.meta = nullptr;  // every group walks from its root, targets in Morton order

@@ -33,6 +33,7 @@
 #include <mutex>
 
 #include "gcs_internal.h"
+#include "pdl.cuh"
 
 namespace gcs {
 namespace {
@@ -68,8 +69,10 @@ uint32_t* g_scratch_addr[kMaxDevices] = {};
 // accumulates for its own sort).
 __global__ void key_histograms_kernel(const uint64_t* __restrict__ keys, int64_t n, uint32_t* __restrict__ hist) {
     __shared__ uint32_t s[kKeyPasses][kRadix];
+    let_next_start();
     for (int t = threadIdx.x; t < kKeyPasses * kRadix; t += blockDim.x) (&s[0][0])[t] = 0u;
     __syncthreads();
+    wait_for_previous();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t k = __ldg(keys + i);
 #pragma unroll
@@ -127,7 +130,7 @@ extern "C" int gcs_sort_pairs_static(uint64_t* keys, uint32_t* vals, uint64_t* k
     int64_t grid = (n + 255) / 256;
     const int64_t cap = (int64_t)current_sm_count() * 8;  // 8 resident 256-thread blocks per SM
     if (grid > cap) grid = cap;
-    key_histograms_kernel<<<(unsigned)grid, 256, 0, st>>>(keys, n, hist);
+    launch_after(key_histograms_kernel, (unsigned)grid, 256, 0, st, keys, n, hist);
     Layout L;
     L.n = (int32_t)n;
     L.nseg = 1;
