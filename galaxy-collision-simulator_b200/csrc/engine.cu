@@ -48,6 +48,7 @@ struct gcs_ctx {
     uint64_t* keys[2] = {nullptr, nullptr};
     uint32_t* idx[2] = {nullptr, nullptr};
     int sorted_buf = 0;
+    bool scratch_zeroed = false;  // within run_stages: the accumulated scratch is already zero
     bool front = false;  // small scenarios sort in one launch (k_front.cu)
     BvhNodeTraverse* tr = nullptr;
     BvhNodeBuild* bd = nullptr;
@@ -201,11 +202,11 @@ int seg_passes(int nseg) { return nseg <= 1 ? 0 : (nseg <= 256 ? 1 : 2); }
 // Byte offsets of the scratch regions for n particles in nseg segments.
 ScratchLayout scratch_layout(int32_t max_segments, int64_t n, int nseg) {
     ScratchLayout s;
-    s.hist = 0;
-    s.walk_q = round256(sizeof(uint32_t) * kMaxPasses * kRadix);
-    s.agg_q = s.walk_q + 128;
-    s.bounds = s.walk_q + 256;
-    s.tiles = s.bounds + round256(sizeof(uint32_t) * 2 * (size_t)max_segments);
+    s.walk_q = 0;
+    s.agg_q = 128;
+    s.bounds = 256;
+    s.hist = s.bounds + round256(sizeof(uint32_t) * 2 * (size_t)max_segments);
+    s.tiles = s.hist + round256(sizeof(uint32_t) * kMaxPasses * kRadix);
     s.lookback = s.tiles + 256;
     s.end = s.lookback + sizeof(uint32_t) * sort_lookback_words(n, kKeyPasses + seg_passes(nseg));
     return s;
@@ -518,19 +519,21 @@ static int run_stage(gcs_ctx* c, const gcs_params* p, int stage, bool gather_bes
         case GCS_STAGE_BOUNDS: {
             if (p->bounds_mode == GCS_BOUNDS_DEVICE) {
                 uint32_t* enc = scratch_at<uint32_t>(c, sl.bounds);
-                GCS_CUDA(c, cudaMemsetAsync(enc, 0, sizeof(uint32_t) * 2 * (size_t)c->nseg, st));
+                if (!c->scratch_zeroed)
+                    GCS_CUDA(c, cudaMemsetAsync(enc, 0, sizeof(uint32_t) * 2 * (size_t)c->nseg, st));
                 launch_bounds(L, c->pos[c->cur], c->chunks, c->n_chunks, enc, c->status, st);
                 launch_bounds_decode(enc, c->seg_bounds, c->nseg, st);
             }
             return check_launch(c, "bounds");
         }
         case GCS_STAGE_ENCODE:
-            GCS_CUDA(c, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kRadix * (size_t)passes, st));
+            if (!c->scratch_zeroed)
+                GCS_CUDA(c, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kRadix * (size_t)passes, st));
             launch_encode(L, c->pos[c->cur], p->bounds_mode, p->global_min, p->global_max,
                           c->seg_bounds, c->keys[0], c->idx[0], hist, seg_passes(c->nseg), st);
             return check_launch(c, "encode");
         case GCS_STAGE_SORT: {
-            GCS_CUDA(c, cudaMemsetAsync(c->scratch + sl.tiles, 0, sl.end - sl.tiles, st));
+            if (!c->scratch_zeroed) GCS_CUDA(c, cudaMemsetAsync(c->scratch + sl.tiles, 0, sl.end - sl.tiles, st));
             for (int pass = 0; pass < passes; ++pass) {
                 const int in = pass & 1;
                 launch_sort_pass(L, pass, c->keys[in], c->idx[in], c->keys[in ^ 1], c->idx[in ^ 1],
@@ -634,7 +637,18 @@ static int run_stages(gcs_ctx* c, const gcs_params* p, int first, int last) {
         if (rc) return rc;
         s = GCS_STAGE_GATHER;
     }
+    // one memset for what bounds, encode and sort accumulate into
+    c->scratch_zeroed = s == GCS_STAGE_BOUNDS && last >= GCS_STAGE_SORT;
+    if (c->scratch_zeroed) {
+        const ScratchLayout sl = scratch_layout(c->max_segments, c->n, c->nseg);
+        const cudaError_t e = cudaMemsetAsync(c->scratch + sl.bounds, 0, sl.end - sl.bounds, c->stream);
+        if (e != cudaSuccess) {
+            set_error(c, "cudaMemsetAsync", e);
+            return GCS_ERR_CUDA;
+        }
+    }
     for (; s <= last; ++s) {
+        if (s > GCS_STAGE_SORT) c->scratch_zeroed = false;
         rc = run_stage(c, p, s, gather_beside_build, kick_in_walk);
         if (rc) return rc;
     }

@@ -95,14 +95,15 @@ struct Layout {
 
 // Per-step scratch, one device allocation.  Each stage zeroes only the
 // region it accumulates into, so any stage can be run on its own:
-//   hist      u32[kMaxPasses][256]  radix digit histograms   (zeroed by encode)
 //   walk_q    u32[2]                walk work queue          (self-resetting)
 //   agg_q     u32                   aggregation block ticket (zeroed by build)
 //   bounds    u32[2 * max_segments] ordered min/max          (zeroed by bounds)
+//   hist      u32[kMaxPasses][256]  radix digit histograms   (zeroed by encode)
 //   tiles     u32[kMaxPasses]       onesweep tile tickets    (zeroed by sort,
 //   lookback  u32[passes][tiles + groups][256] decoupled look-back, with lookback)
+// A run of all three stages zeroes bounds .. lookback at once.
 struct ScratchLayout {
-    size_t hist, walk_q, agg_q, bounds, tiles, lookback, end;
+    size_t walk_q, agg_q, bounds, hist, tiles, lookback, end;
 };
 
 // ---- launchers (one per stage; all asynchronous on `st`) ----------------

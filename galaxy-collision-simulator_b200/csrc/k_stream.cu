@@ -9,6 +9,7 @@
 
 #include "gcs_internal.h"
 #include "device_math.cuh"
+#include "digits.cuh"
 #include "pdl.cuh"
 
 namespace gcs {
@@ -164,7 +165,8 @@ __global__ void bounds_decode_kernel(const uint32_t* __restrict__ enc, float2* _
 // digits, plus the segment-id digits when there is more than one segment)
 // are accumulated here in shared memory, so the sort needs no separate
 // counting pass over the keys.
-__global__ void encode_kernel(Layout L, const float4* __restrict__ pos, int bounds_mode,
+__global__ void __launch_bounds__(kCountThreads, 2)
+encode_kernel(Layout L, const float4* __restrict__ pos, int bounds_mode,
                               float gmin, float gmax, const float2* __restrict__ seg_bounds,
                               uint64_t* __restrict__ keys, uint32_t* __restrict__ idx,
                               uint32_t* __restrict__ hist, int n_seg_passes) {
@@ -177,24 +179,29 @@ __global__ void encode_kernel(Layout L, const float4* __restrict__ pos, int boun
     float lo = gmin, scale = 0.0f;
     int cur_seg = -1;
     if (bounds_mode == GCS_BOUNDS_CALLER) scale = morton_scale(gmin, gmax);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < L.n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 p = __ldg(pos + i);
-        const int seg = (L.nseg > 1) ? __ldg(L.seg_id + i) : 0;
-        if (bounds_mode != GCS_BOUNDS_CALLER && seg != cur_seg) {
-            const float2 b = __ldg(seg_bounds + seg);
-            lo = b.x;
-            scale = morton_scale(b.x, b.y);
-            cur_seg = seg;
+    // whole warps go round together (count_digits)
+    for (int base = blockIdx.x * kCountThreads + (threadIdx.x & ~31); base < L.n; base += gridDim.x * kCountThreads) {
+        const int i = base + (threadIdx.x & 31);
+        const bool valid = i < L.n;
+        uint64_t k = 0ull;
+        int seg = 0;
+        if (valid) {
+            const float4 p = __ldg(pos + i);
+            seg = (L.nseg > 1) ? __ldg(L.seg_id + i) : 0;
+            if (bounds_mode != GCS_BOUNDS_CALLER && seg != cur_seg) {
+                const float2 b = __ldg(seg_bounds + seg);
+                lo = b.x;
+                scale = morton_scale(b.x, b.y);
+                cur_seg = seg;
+            }
+            k = morton63(p.x, p.y, p.z, lo, scale);
+            keys[i] = k;
+            idx[i] = (uint32_t)i;
         }
-        const uint64_t k = morton63(p.x, p.y, p.z, lo, scale);
-        keys[i] = k;
-        idx[i] = (uint32_t)i;
-#pragma unroll
-        for (int d = 0; d < kKeyPasses; ++d)
-            atomicAdd(&s_hist[d][(uint32_t)(k >> (kRadixBits * d)) & (kRadix - 1)], 1u);
-        for (int d = 0; d < n_seg_passes; ++d)
-            atomicAdd(&s_hist[kKeyPasses + d][((uint32_t)seg >> (kRadixBits * d)) & (kRadix - 1)], 1u);
+        count_digits(s_hist, k, valid);
+        if (valid)
+            for (int d = 0; d < n_seg_passes; ++d)
+                atomicAdd(&s_hist[kKeyPasses + d][((uint32_t)seg >> (kRadixBits * d)) & (kRadix - 1)], 1u);
     }
     __syncthreads();
     for (int t = threadIdx.x; t < passes * kRadix; t += blockDim.x) {
@@ -434,7 +441,7 @@ void launch_encode(const Layout& L, const float4* pos, int bounds_mode, float gm
                    const float2* seg_bounds, uint64_t* keys, uint32_t* idx, uint32_t* hist,
                    int n_seg_passes, cudaStream_t st) {
     if (L.n <= 0) return;
-    launch_after(encode_kernel, stream_grid(L.n), kStreamThreads, 0, st, L, pos, bounds_mode, gmin, gmax, seg_bounds,
+    launch_after(encode_kernel, count_grid(L.n, current_sm_count()), kCountThreads, 0, st, L, pos, bounds_mode, gmin, gmax, seg_bounds,
                  keys, idx, hist, n_seg_passes);
 }
 

@@ -32,6 +32,7 @@
 #include <cstdio>
 #include <mutex>
 
+#include "digits.cuh"
 #include "gcs_internal.h"
 #include "pdl.cuh"
 
@@ -67,16 +68,17 @@ uint32_t* g_scratch_addr[kMaxDevices] = {};
 
 // Digit histograms of all 8 key digits (what the engine's encode kernel
 // accumulates for its own sort).
-__global__ void key_histograms_kernel(const uint64_t* __restrict__ keys, int64_t n, uint32_t* __restrict__ hist) {
+__global__ void __launch_bounds__(kCountThreads, 2)
+key_histograms_kernel(const uint64_t* __restrict__ keys, int64_t n, uint32_t* __restrict__ hist) {
     __shared__ uint32_t s[kKeyPasses][kRadix];
     let_next_start();
     for (int t = threadIdx.x; t < kKeyPasses * kRadix; t += blockDim.x) (&s[0][0])[t] = 0u;
     __syncthreads();
     wait_for_previous();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = __ldg(keys + i);
-#pragma unroll
-        for (int d = 0; d < kKeyPasses; ++d) atomicAdd(&s[d][(uint32_t)(k >> (kRadixBits * d)) & (kRadix - 1)], 1u);
+    for (int64_t base = (int64_t)blockIdx.x * kCountThreads + (threadIdx.x & ~31); base < n;
+         base += (int64_t)gridDim.x * kCountThreads) {
+        const int64_t i = base + (threadIdx.x & 31);
+        count_digits(s, i < n ? __ldg(keys + i) : 0ull, i < n);
     }
     __syncthreads();
     for (int t = threadIdx.x; t < kKeyPasses * kRadix; t += blockDim.x) {
@@ -127,10 +129,7 @@ extern "C" int gcs_sort_pairs_static(uint64_t* keys, uint32_t* vals, uint64_t* k
     uint32_t* lookback = own_status + kStatusWords;
     const size_t clear_words = kHistWords + kTicketWords + kStatusWords + sort_lookback_words(n, kKeyPasses);
     if (cudaMemsetAsync(base, 0, clear_words * sizeof(uint32_t), st) != cudaSuccess) return GCS_ERR_CUDA;
-    int64_t grid = (n + 255) / 256;
-    const int64_t cap = (int64_t)current_sm_count() * 8;  // 8 resident 256-thread blocks per SM
-    if (grid > cap) grid = cap;
-    launch_after(key_histograms_kernel, (unsigned)grid, 256, 0, st, keys, n, hist);
+    launch_after(key_histograms_kernel, count_grid(n, current_sm_count()), kCountThreads, 0, st, keys, n, hist);
     Layout L;
     L.n = (int32_t)n;
     L.nseg = 1;
