@@ -571,7 +571,7 @@ static int run_stage(gcs_ctx* c, const gcs_params* p, int stage, bool gather_bes
         case GCS_STAGE_AGGREGATE: {
             const WalkNodeParams wnp = walk_node_params(c, p);
             uint32_t* ticket = scratch_at<uint32_t>(c, sl.agg_q);
-            if (!c->relay_empty) launch_relay_reset(L, c->tr, c->wn, c->com64, ticket, st);
+            if (!c->relay_empty) launch_relay_reset(L, c->tr, c->bd, c->wn, c->com64, ticket, st);
             c->relay_empty = false;
             launch_aggregate(L, c->pos[c->cur], c->tr, c->bd, c->com64, c->leaf_parent, p->com_fp64, wnp,
                              reinterpret_cast<int2*>(c->keys[c->sorted_buf ^ 1]), c->idx[c->sorted_buf ^ 1], ticket,

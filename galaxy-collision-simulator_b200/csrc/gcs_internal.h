@@ -149,16 +149,16 @@ void launch_gather(const uint32_t* idx, const float4* pos_in, const float4* vel_
                    float4* vel_out, int64_t n, cudaStream_t st);
 struct WalkNode;
 struct WalkNodeParams;
-// The build also empties the aggregation's relay (k_tree.cu: words of wn, tr
-// and com64 of the nodes above its blocks) and zeroes its block ticket; an
+// The build also empties the aggregation's relay (k_tree.cu: words of wn,
+// tr, bd and com64 of the nodes above its blocks) and zeroes its block ticket; an
 // aggregation that does not follow a build needs launch_relay_reset first.
 // roots, n_roots: the aggregation's lists between its two launches, n records
 // each (the sort's spare key and index buffers).
 void launch_build(const Layout& L, const uint64_t* keys, BvhNodeTraverse* tr, BvhNodeBuild* bd,
                   int32_t* leaf_parent, WalkNode* wn, double4* com64, uint32_t* agg_ticket, uint32_t* status,
                   cudaStream_t st);
-void launch_relay_reset(const Layout& L, BvhNodeTraverse* tr, WalkNode* wn, double4* com64, uint32_t* agg_ticket,
-                        cudaStream_t st);
+void launch_relay_reset(const Layout& L, BvhNodeTraverse* tr, BvhNodeBuild* bd, WalkNode* wn, double4* com64,
+                        uint32_t* agg_ticket, cudaStream_t st);
 void launch_aggregate(const Layout& L, const float4* pos, BvhNodeTraverse* tr, BvhNodeBuild* bd,
                       double4* com64, const int32_t* leaf_parent, int com_fp64, const WalkNodeParams& wnp,
                       int2* roots, uint32_t* n_roots, uint32_t* agg_ticket, uint32_t* status, cudaStream_t st);
@@ -176,7 +176,7 @@ struct WalkParams {
 //   link  bits(width^2), code_a, code_b, 0 where
 //           code_b >= kWalkBucketTag  the node holds <= L particles, summed
 //                                     directly: [code_a, code_a + code_b - tag)
-//           code_b == kWalkSkipTag    malformed links: nothing below it
+//           code_b == kWalkSkipTag    malformed links: a bucket of none
 //           otherwise                 children: >= 0 internal node,
 //                                     < 0 particle ~code
 // Every code names an index below the context's capacity, so a walk over
@@ -187,7 +187,7 @@ struct WalkNode {
 };
 static_assert(sizeof(WalkNode) == 32, "WalkNode must be 32 bytes");
 constexpr int kWalkBucketTag = 1 << 30;
-constexpr int kWalkSkipTag = 0x7FFFFFFF;
+constexpr int kWalkSkipTag = kWalkBucketTag;
 // G and leaf size of the walk records an aggregation writes.
 struct WalkNodeParams {
     WalkNode* wn;

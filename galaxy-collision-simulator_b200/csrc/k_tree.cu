@@ -38,9 +38,12 @@ constexpr int kAggMaxLevels = 96;    // internal levels of a valid tree (strictl
 // A node whose particles lie in more than one block's run (aggregate_kernel)
 // is computed by its right child's climber, which gets the left child's
 // values from the node's own records, before they hold the node's values:
-//   wn     lo.x lo.y lo.z hi.x | hi.y hi.z com.x com.y     (32-bit words)
-//   tr     com.z mass
-//   com64  the FP64 sums, of a left child that has them    (64-bit words)
+//   wn     lo.x lo.y lo.z hi.x       (32-bit words, in place of cm)
+//   tr     hi.y hi.z com.x com.y     (in place of com and mass)
+//   bd     com.z mass                (in place of min x and y)
+//   com64  the FP64 sums, of a left child that has them (64-bit words)
+// (never in place of a walk record's codes: a walk that follows a failed
+// climb must still read inside its arrays)
 // The build (or launch_relay_reset) sets every word of these to all ones, the
 // left child's climber writes them, and a word that is not all ones is there:
 // each is a single relaxed access and needs no fence, counter or order among
@@ -80,12 +83,12 @@ __device__ __forceinline__ unsigned long long relay_word(double f) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(f);
     return u == ~0ull ? 0x7FFFFFFFFFFFFFFFull : u;
 }
-__device__ __forceinline__ void relay_clear(WalkNode* wn, BvhNodeTraverse* tr, double4* com64, int node) {
+__device__ __forceinline__ void relay_clear(WalkNode* wn, BvhNodeTraverse* tr, BvhNodeBuild* bd, double4* com64,
+                                            int node) {
     const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
-    uint4* w = reinterpret_cast<uint4*>(wn + node);
-    w[0] = ones;
-    w[1] = ones;
-    *reinterpret_cast<uint2*>(tr + node) = make_uint2(~0u, ~0u);
+    *reinterpret_cast<uint4*>(wn + node) = ones;
+    *reinterpret_cast<uint4*>(tr + node) = ones;
+    *reinterpret_cast<uint2*>(bd + node) = make_uint2(~0u, ~0u);
     uint4* q = reinterpret_cast<uint4*>(com64 + node);
     q[0] = ones;
     q[1] = ones;
@@ -158,7 +161,7 @@ __global__ void build_kernel(Layout L, const uint64_t* __restrict__ keys,
         else bd[cr].parent = node;
         bd[node].flag = 0;
         if (i == 0) bd[node].parent = -1;       // segment root
-        if (above_blocks(off + lo, off + hi)) relay_clear(wn, tr, com64, node);
+        if (above_blocks(off + lo, off + hi)) relay_clear(wn, tr, bd, com64, node);
     }
 }
 
@@ -453,12 +456,11 @@ struct RelayWords {
     uint2 w2;
     ulonglong2 q0, q1;
 };
-__device__ __forceinline__ void relay_load(const WalkNode* wn, const BvhNodeTraverse* tr, const double4* com64,
-                                           const RiseNode& n, RelayWords& r) {
-    const uint4* w = reinterpret_cast<const uint4*>(wn + n.node);
-    r.w0 = load_relaxed(w);
-    r.w1 = load_relaxed(w + 1);
-    r.w2 = load_relaxed2(tr + n.node);
+__device__ __forceinline__ void relay_load(const WalkNode* wn, const BvhNodeTraverse* tr, const BvhNodeBuild* bd,
+                                           const double4* com64, const RiseNode& n, RelayWords& r) {
+    r.w0 = load_relaxed(wn + n.node);
+    r.w1 = load_relaxed(tr + n.node);
+    r.w2 = load_relaxed2(bd + n.node);
     r.q0 = r.q1 = make_ulonglong2(0ull, 0ull);
     if (n.big_l) {
         r.q0 = load_relaxed64(com64 + n.node);
@@ -482,13 +484,13 @@ __device__ __forceinline__ ChildData relay_values(const RelayWords& r) {
     return A;
 }
 // The values of node n's left child, to its right child's climber.
-__device__ __forceinline__ void hand_over(WalkNode* wn, BvhNodeTraverse* tr, double4* com64, const RiseNode& n,
-                                          const ChildData& c) {
-    uint4* w = reinterpret_cast<uint4*>(wn + n.node);
-    store_relaxed(w, make_uint4(relay_word(c.lo.x), relay_word(c.lo.y), relay_word(c.lo.z), relay_word(c.hi.x)));
-    store_relaxed(w + 1, make_uint4(relay_word(c.hi.y), relay_word(c.hi.z), relay_word(c.com.x),
-                                    relay_word(c.com.y)));
-    store_relaxed(reinterpret_cast<uint2*>(tr + n.node), make_uint2(relay_word(c.com.z), relay_word(c.m)));
+__device__ __forceinline__ void hand_over(WalkNode* wn, BvhNodeTraverse* tr, BvhNodeBuild* bd, double4* com64,
+                                          const RiseNode& n, const ChildData& c) {
+    store_relaxed(reinterpret_cast<uint4*>(wn + n.node),
+                  make_uint4(relay_word(c.lo.x), relay_word(c.lo.y), relay_word(c.lo.z), relay_word(c.hi.x)));
+    store_relaxed(reinterpret_cast<uint4*>(tr + n.node),
+                  make_uint4(relay_word(c.hi.y), relay_word(c.hi.z), relay_word(c.com.x), relay_word(c.com.y)));
+    store_relaxed(reinterpret_cast<uint2*>(bd + n.node), make_uint2(relay_word(c.com.z), relay_word(c.m)));
     if (n.big_l) {
         ulonglong2* q = reinterpret_cast<ulonglong2*>(com64 + n.node);
         store_relaxed(q, make_ulonglong2(relay_word(c.mx.x), relay_word(c.mx.y)));
@@ -543,11 +545,11 @@ rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restric
         RiseNode N = rise_node(tr, bd, node, s, ni, fp64);
         bool ok = N.node >= 0 && valid_links(N, from, lim);
         if (ok && N.cl == from) {
-            hand_over(wnp.wn, tr, com64, N, mine);
+            hand_over(wnp.wn, tr, bd, com64, N, mine);
             continue;
         }
         RelayWords w;
-        if (ok) relay_load(wnp.wn, tr, com64, N, w);
+        if (ok) relay_load(wnp.wn, tr, bd, com64, N, w);
         RiseNode up = rise_node(tr, bd, ok ? N.up : -1, s, ni, fp64);
         uint32_t polls = 0;
         int levels = 0;
@@ -556,7 +558,7 @@ rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restric
         while (ok) {
             if (!relay_there(w)) {
                 ok = ++polls < kRelayPolls;
-                relay_load(wnp.wn, tr, com64, N, w);
+                relay_load(wnp.wn, tr, bd, com64, N, w);
                 continue;
             }
             const ChildData A = relay_values(w);
@@ -583,10 +585,10 @@ rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restric
             ok = !more ? cur.up < 0 : valid_links(up, cur.node, lim) && ++levels <= kAggMaxLevels;
             const bool hand = ok && more && up.cl == cur.node;
             if (sums && ok && more && !(hand ? up.big_l : up.big_r)) ok = false;  // FP64 nodes have FP64 parents
-            if (hand && ok) hand_over(wnp.wn, tr, com64, up, next);
+            if (hand && ok) hand_over(wnp.wn, tr, bd, com64, up, next);
             N = up;
             if (ok && more && !hand) {
-                relay_load(wnp.wn, tr, com64, N, w);
+                relay_load(wnp.wn, tr, bd, com64, N, w);
                 up = rise_node(tr, bd, N.up, s, ni, fp64);
             }
             if (sums)
@@ -611,8 +613,9 @@ rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restric
 // Empty relay words of every node above the blocks, and the block ticket, for
 // an aggregation that does not follow a build (one thread per particle, as in
 // walk_nodes_kernel).
-__global__ void relay_reset_kernel(Layout L, BvhNodeTraverse* __restrict__ tr, WalkNode* __restrict__ wn,
-                                   double4* __restrict__ com64, uint32_t* __restrict__ ticket) {
+__global__ void relay_reset_kernel(Layout L, BvhNodeTraverse* __restrict__ tr, BvhNodeBuild* __restrict__ bd,
+                                   WalkNode* __restrict__ wn, double4* __restrict__ com64,
+                                   uint32_t* __restrict__ ticket) {
     let_next_start();
     wait_for_previous();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -621,7 +624,7 @@ __global__ void relay_reset_kernel(Layout L, BvhNodeTraverse* __restrict__ tr, W
     const int s = L.nseg > 1 ? __ldg(L.seg_id + g) : 0;
     if (g + 1 >= (int)__ldg(L.seg_off + s + 1)) return;
     const int re = tr[g - s].range_end;
-    if (above_blocks(min(g, re), max(g, re))) relay_clear(wn, tr, com64, g - s);
+    if (above_blocks(min(g, re), max(g, re))) relay_clear(wn, tr, bd, com64, g - s);
 }
 
 int tree_grid(int64_t n) {
@@ -638,10 +641,10 @@ void launch_build(const Layout& L, const uint64_t* keys, BvhNodeTraverse* tr, Bv
     launch_after(build_kernel, tree_grid(L.n), 256, 0, st, L, keys, tr, bd, leaf_parent, wn, com64, agg_ticket, status);
 }
 
-void launch_relay_reset(const Layout& L, BvhNodeTraverse* tr, WalkNode* wn, double4* com64, uint32_t* agg_ticket,
-                        cudaStream_t st) {
+void launch_relay_reset(const Layout& L, BvhNodeTraverse* tr, BvhNodeBuild* bd, WalkNode* wn, double4* com64,
+                        uint32_t* agg_ticket, cudaStream_t st) {
     if (L.n <= 0) return;
-    launch_after(relay_reset_kernel, tree_grid(L.n), 256, 0, st, L, tr, wn, com64, agg_ticket);
+    launch_after(relay_reset_kernel, tree_grid(L.n), 256, 0, st, L, tr, bd, wn, com64, agg_ticket);
 }
 
 void launch_aggregate(const Layout& L, const float4* pos, BvhNodeTraverse* tr, BvhNodeBuild* bd,
