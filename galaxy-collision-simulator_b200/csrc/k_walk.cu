@@ -13,6 +13,16 @@
 // With theta = 1 and L = 1 every target sees exactly the reference's set of
 // terms; only the order of the FP32 sums differs.
 //
+// What bounds it: instruction issue (75 % of the issue slots; FMA pipe 52 %,
+// ALU 47 %).  Half of the instructions are the traversal's, so what a round
+// spends besides its terms counts: with the group's box in shared memory, one
+// population count a node for its list slot, one word a node for its pushes
+// and sources, ballots masked by the node's owner and the sources' nodes found
+// by one reduction, the walk stage went from 2,420 to 2,277 us at 1,048,576
+// particles (theta 0.5, leaf 4), 1,016 to 935 at 777,777 (0.7, leaf 8), 4,977
+// to 4,795 at 2,000,000 with potentials and 2,800 to 2,525 at 1,000,000 in
+// 64-target groups, bit for bit the same.
+//
 // Execution: a persistent grid of warps pulls groups of <= 32*T consecutive
 // (Morton-adjacent) targets of one segment from a global work queue; lane l
 // holds targets l and l+32 (T = 2) of its group.  The warp walks the tree once
@@ -173,6 +183,7 @@ struct WarpSmem {
     float4 sxy[kSrcCap / 2];        // particle sources in pairs: x0 x1 y0 y1
     float4 szm[kSrcCap / 2];        // z0 z1 Gm0 Gm1
     uint2 smask[T][kSrcCap / 2];    // lane masks
+    float4 box[2];                  // the group's bounding box
     int srcp[kSrcCap];              // the list before its fetch: particle
     uint32_t srcm[T][kSrcCap];      //   and its lane masks
 };
@@ -191,12 +202,13 @@ __device__ __forceinline__ void put_mask(uint2* mk, int slot, uint32_t mask) {
     reinterpret_cast<uint32_t*>(mk + (slot >> 1))[slot & 1] = mask;
 }
 
-// Resident blocks per SM the register budget is set for (T=1: H=1 48
-// registers a thread, 40 warps; H=2 64 registers, 32 warps; T=2: 80
-// registers, 24 warps).
+// Resident blocks per SM the register budget is set for (T=1: 64 registers a
+// thread, 32 warps; T=2: 80 registers, 24 warps).  H=1 with five blocks (48
+// registers, spills) 976 against 968 us at 777,777 particles, theta 0.7; T=2
+// with two and four blocks 2,626 and 2,660 against 2,551 us at 1,000,000.
 template <int H, int T>
 struct WalkOcc {
-    static constexpr int kMinBlocks = T == 2 ? 3 : (H == 1 ? 5 : 4);
+    static constexpr int kMinBlocks = T == 2 ? 3 : 4;
 };
 
 // Sums of one target: two partial sums per component (even / odd slots).
@@ -277,10 +289,22 @@ struct Targets {
 
 // Sum the listed particle sources into every target whose lane bit is in
 // the source's mask for its slot (leaf rule: skip d2 <= 1.01 eps^2).
+// Unrolling of the evaluation loops, in pairs of list slots.  Walk stage in us
+// at 1,048,576 particles (T = 1) / 1,000,000 in 64-target groups (T = 2): mixed
+// loop by 2 2,371 / 2,711, by 4 2,346 / 2,857; source loop by 4 2,371 / 2,711,
+// by 2 2,375 / 2,546 (T = 2 loops are twice as long and leave the instruction
+// cache); take loops by 2 and 8 within 0.2 % for T = 1, by 2 1.6 % slower for
+// T = 2.
+template <int T>
+struct Unroll {
+    static constexpr int kList = 4, kFull = 4, kTake = 4, kMixed = T == 1 ? 4 : 2, kSrc = T == 1 ? 4 : 2;
+};
+
 template <int H, int T, bool kPot, bool kCount>
 __device__ __forceinline__ void flush_sources(WarpSmem<H, T>& W, int nsrc, int lane, uint32_t lane_bit,
                                               const float4* __restrict__ pos, float G, const Targets<T>& X,
                                               float2 e2, float leaf_thr, Accum (&A)[T], WarpCount& WC) {
+    using U = Unroll<T>;
     __syncwarp();
     const int padded = (nsrc + 1) & ~1;
     for (int e = lane; e < padded; e += 32) {
@@ -299,7 +323,7 @@ __device__ __forceinline__ void flush_sources(WarpSmem<H, T>& W, int nsrc, int l
         for (int t = 0; t < T; ++t) put_mask(W.smask[t], e, m[t]);
     }
     __syncwarp();
-#pragma unroll 4
+#pragma unroll(U::kSrc)
     for (int q = 0; q < (padded >> 1); ++q) {
         const float4 zm = W.szm[q];
         const float4 xy = W.sxy[q];
@@ -376,6 +400,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
             uint32_t* __restrict__ status, unsigned long long* __restrict__ counts,
             typename EntryOf<T>::type* __restrict__ gstack, int gstack_cap, WalkEpilogue ep,
             WalkFrontier fr) {
+    using U = Unroll<T>;
     using Smem = WarpSmem<H, T>;
     using Entry = typename Smem::Entry;
     extern __shared__ __align__(16) unsigned char walk_smem[];
@@ -434,6 +459,10 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
             box_hi.y = fmaxf(box_hi.y, __shfl_xor_sync(kFull, box_hi.y, o));
             box_hi.z = fmaxf(box_hi.z, __shfl_xor_sync(kFull, box_hi.z, o));
         }
+        if (lane == 0) {
+            W.box[0] = make_float4(box_lo.x, box_lo.y, box_lo.z, 0.f);
+            W.box[1] = make_float4(box_hi.x, box_hi.y, box_hi.z, 0.f);
+        }
         const int s = grp.seg;
         const int off = (int)__ldg(L.seg_off + s);
         const int seg_n = (int)__ldg(L.seg_off + s + 1) - off;
@@ -461,7 +490,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                         put_pair(W.sxy, W.szm, e, q);
                     }
                     __syncwarp();
-#pragma unroll 4
+#pragma unroll(U::kList)
                     for (int q = 0; q < (padded >> 1); ++q) {
                         const float4 zm = W.szm[q];
                         const float4 xy = W.sxy[q];
@@ -530,6 +559,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                     break;
                 }
                 top -= b;
+                const float4 blo = W.box[0], bhi = W.box[1];
                 // 1-2. fetch and classify nodes lane and lane+32
                 int code_a[H], code_b[H], cls[H];
                 uint32_t my_mask[H][T];
@@ -558,7 +588,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                         bool full = true;
 #pragma unroll
                         for (int t = 0; t < T; ++t) full = full && my_mask[h][t] == live[t];
-                        cls[h] = box_class(a, w2[h], box_lo, box_hi, eps2, k_take, k_open);
+                        cls[h] = box_class(a, w2[h], make_float3(blo.x, blo.y, blo.z), make_float3(bhi.x, bhi.y, bhi.z), eps2, k_take, k_open);
                         if (cls[h] == kClassTake && full) cls[h] = kClassTakeFull;
                     }
                 }
@@ -584,9 +614,10 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                     int full_before = 0, take_before = 0, mixed_before = 0;
 #pragma unroll
                     for (int h = 0; h < H; ++h) {
-                        slot[h] = cls[h] == kClassTakeFull ? full_before + __popc(bf[h] & lt)
-                                : cls[h] == kClassTake ? take_base + take_before + __popc(bt[h] & lt)
-                                : cls[h] == kClassMixed ? mixed_base + mixed_before + __popc(bm[h] & lt) : -1;
+                        const bool f = cls[h] == kClassTakeFull, k = cls[h] == kClassTake, m = cls[h] == kClassMixed;
+                        const uint32_t of_class = f ? bf[h] : k ? bt[h] : bm[h];
+                        const int at = f ? full_before : k ? take_base + take_before : mixed_base + mixed_before;
+                        slot[h] = f || k || m ? at + __popc(of_class & lt) : -1;
                         full_before += __popc(bf[h]);
                         take_before += __popc(bt[h]);
                         mixed_before += __popc(bm[h]);
@@ -598,9 +629,9 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                         }
                     }
                     const float4 empty = make_float4(1e30f, 1e30f, 1e30f, 0.0f);
-                    const int pad = lane == 0 ? ((n_full & 1) ? n_full : -1)
-                                  : lane == 1 ? ((n_take & 1) ? take_base + n_take : -1)
-                                  : lane == 2 ? ((n_mixed & 1) ? mixed_base + n_mixed : -1) : -1;
+                    // lane l pads list l where it is odd
+                    const int end = lane == 0 ? n_full : lane == 1 ? take_base + n_take : mixed_base + n_mixed;
+                    const int pad = lane < 3 && (end & 1) ? end : -1;  // (lists start at even slots)
                     if (pad >= 0) {
                         put_pair(W.pxy, W.pzm, pad, empty);
 #pragma unroll
@@ -629,7 +660,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                 }
                 // 3a. nodes every live target accepts: monopole terms, two
                 // nodes per packed evaluation, no masks
-#pragma unroll 4
+#pragma unroll(U::kFull)
                 for (int q = 0; q < (take_base >> 1); ++q) {
                     const float4 zm = W.pzm[q];
                     const float4 xy = W.pxy[q];
@@ -645,7 +676,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                         if (valid[t]) A[t].n_mono += (uint32_t)n_full;
                 }
                 // 3b. nodes accepted by every target of their masks
-#pragma unroll 4
+#pragma unroll(U::kTake)
                 for (int q = take_base >> 1; q < (mixed_base >> 1); ++q) {
                     const float4 zm = W.pzm[q];
                     const float4 xy = W.pxy[q];
@@ -660,7 +691,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                 }
                 // 3c. mixed nodes: each target's own test; lane 0 records the
                 // ballots of opening lanes for the nodes' owners
-#pragma unroll 2
+#pragma unroll(U::kMixed)
                 for (int q = mixed_base >> 1; q < ((mixed_base + n_mixed + 1) >> 1); ++q) {
                     const float4 zm = W.pzm[q];
                     const float4 xy = W.pxy[q];
@@ -678,16 +709,18 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                             WC.l_accept += (uint32_t)(__popc(__ballot_sync(kFull, act0 && take0)) +
                                                       __popc(__ballot_sync(kFull, act1 && take1)));
                         }
-                        const uint32_t om0 = __ballot_sync(kFull, act0 && !take0);
-                        const uint32_t om1 = __ballot_sync(kFull, act1 && !take1);
+                        const uint32_t om0 = __ballot_sync(kFull, !take0);
+                        const uint32_t om1 = __ballot_sync(kFull, !take1);
                         if (lane == 0) W.pnopen[t][q] = make_uint2(om0, om1);
                     }
                 }
                 __syncwarp();
                 // 4. parallel push / append for the opened nodes
                 uint32_t my_open[H][T];
-                int n_push[H], n_src[H];
-                int lane_push = 0, lane_src = 0;
+                // pushes << 16 | sources of each node: a bucket's particles, or
+                // its two children, each one or the other
+                uint32_t work[H];
+                uint32_t both = 0u;
 #pragma unroll
                 for (int h = 0; h < H; ++h) {
                     uint32_t any = 0u;
@@ -695,30 +728,22 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                     for (int t = 0; t < T; ++t) {
                         my_open[h][t] = cls[h] == kClassOpen ? my_mask[h][t]
                                       : (cls[h] == kClassMixed
-                                             ? reinterpret_cast<const uint32_t*>(W.pnopen[t])[slot[h]] : 0u);
+                                             ? reinterpret_cast<const uint32_t*>(W.pnopen[t])[slot[h]] & my_mask[h][t] : 0u);
                         any |= my_open[h][t];
                     }
-                    n_push[h] = 0;
-                    n_src[h] = 0;
-                    if (any != 0u && code_b[h] != kWalkSkipTag) {
-                        if (code_b[h] >= kWalkBucketTag) {
-                            n_src[h] = code_b[h] - kWalkBucketTag;
-                        } else {
-                            n_push[h] = (code_a[h] >= 0) + (code_b[h] >= 0);
-                            n_src[h] = (code_a[h] < 0) + (code_b[h] < 0);
-                        }
-                    }
-                    lane_push += n_push[h];
-                    lane_src += n_src[h];
+                    const uint32_t leaves = ((uint32_t)code_a[h] >> 31) + ((uint32_t)code_b[h] >> 31);
+                    work[h] = any == 0u ? 0u
+                            : code_b[h] >= kWalkBucketTag ? (uint32_t)(code_b[h] - kWalkBucketTag)
+                                                          : (2u << 16) - leaves * 0xFFFFu;
+                    both += work[h];
                 }
-                const uint32_t both = ((uint32_t)lane_push << 16) | (uint32_t)lane_src;
                 const uint32_t excl = warp_exclusive_scan(both, lane);
                 const uint32_t total = __shfl_sync(kFull, excl + both, 31);
                 {
                     int at = top + (int)(excl >> 16);
 #pragma unroll
                     for (int h = 0; h < H; ++h) {
-                        if (n_push[h] > 0) {
+                        if ((work[h] >> 16) != 0u) {
                             if (code_a[h] >= 0) W.stk[at++] = make_entry(code_a[h], my_open[h]);
                             if (code_b[h] >= 0) W.stk[at++] = make_entry(code_b[h], my_open[h]);
                         }
@@ -737,54 +762,74 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                     int before = 0, n_desc = 0;
 #pragma unroll
                     for (int h = 0; h < H; ++h) {
-                        const uint32_t bh = __ballot_sync(kFull, n_src[h] > 0);
+                        const uint32_t bh = __ballot_sync(kFull, (work[h] & 0xFFFFu) != 0u);
                         before += __popc(bh & lt);
                         n_desc += __popc(bh);
                     }
+                    uint32_t starts = 0u;  // first sources (of up to 32) of this lane's nodes
                     {
                         int d = before, first = src_at;
 #pragma unroll
                         for (int h = 0; h < H; ++h) {
-                            if (n_src[h] > 0) {
+                            if ((work[h] & 0xFFFFu) != 0u) {
                                 W.sdesc[d] = make_int4(first, code_a[h], code_b[h], 0);
+                                starts |= 1u << (first & 31);
 #pragma unroll
                                 for (int t = 0; t < T; ++t)
                                     reinterpret_cast<uint32_t*>(W.pmask[t])[d] = my_open[h][t];
                                 ++d;
                             }
-                            first += n_src[h];
+                            first += (int)(work[h] & 0xFFFFu);
                         }
                     }
                     __syncwarp();
-                    // the round's sources [0, add), appended in windows that
-                    // fit the list (flushing between windows), one per lane
-                    for (int base = 0; base < add;) {
-                        if (nsrc == kSrcCap) {
-                            flush_sources<H, T, kPot, kCount>(W, nsrc, lane, lane_bit, pos, G, X, e2, leaf_thr, A,
-                                                              WC);
-                            nsrc = 0;
-                        }
-                        const int window = min(kSrcCap - nsrc, add - base);
-                        for (int j = base + lane; j < base + window; j += 32) {
-                            // the last descriptor starting at or before j
-                            int lo = 0, hi = n_desc - 1;
-                            while (lo < hi) {
-                                const int mid = (lo + hi + 1) >> 1;
-                                if (W.sdesc[mid].x <= j) lo = mid;
-                                else hi = mid - 1;
-                            }
-                            const int4 e = W.sdesc[lo];
-                            const int r = j - e.x;  // r-th source of that node
-                            const int particle = e.z >= kWalkBucketTag ? e.y + r
-                                               : ((r == 0 && e.y < 0) ? ~e.y : ~e.z);
-                            const int at = nsrc + (j - base);
-                            W.srcp[at] = particle;
+                    if (add <= 32) {
+                        // one window (fewer than 32 sources are left from the
+                        // last round): lane j's descriptor is the last one
+                        // starting at or before j
+                        starts = __reduce_or_sync(kFull, starts);
+                        if (lane < add) {
+                            const int d = __popc(starts & (lt | lane_bit)) - 1;
+                            const int4 e = W.sdesc[d];
+                            const int r = lane - e.x;  // r-th source of that node
+                            W.srcp[nsrc + lane] = e.z >= kWalkBucketTag ? e.y + r
+                                                : ((r == 0 && e.y < 0) ? ~e.y : ~e.z);
 #pragma unroll
                             for (int t = 0; t < T; ++t)
-                                W.srcm[t][at] = reinterpret_cast<const uint32_t*>(W.pmask[t])[lo];
+                                W.srcm[t][nsrc + lane] = reinterpret_cast<const uint32_t*>(W.pmask[t])[d];
                         }
-                        nsrc += window;
-                        base += window;
+                        nsrc += add;
+                    } else {
+                        // appended in windows that fit the list (flushing
+                        // between windows), one per lane
+                        for (int base = 0; base < add;) {
+                            if (nsrc == kSrcCap) {
+                                flush_sources<H, T, kPot, kCount>(W, nsrc, lane, lane_bit, pos, G, X, e2, leaf_thr, A,
+                                                                  WC);
+                                nsrc = 0;
+                            }
+                            const int window = min(kSrcCap - nsrc, add - base);
+                            for (int j = base + lane; j < base + window; j += 32) {
+                                // the last descriptor starting at or before j
+                                int lo = 0, hi = n_desc - 1;
+                                while (lo < hi) {
+                                    const int mid = (lo + hi + 1) >> 1;
+                                    if (W.sdesc[mid].x <= j) lo = mid;
+                                    else hi = mid - 1;
+                                }
+                                const int4 e = W.sdesc[lo];
+                                const int r = j - e.x;  // r-th source of that node
+                                const int particle = e.z >= kWalkBucketTag ? e.y + r
+                                                   : ((r == 0 && e.y < 0) ? ~e.y : ~e.z);
+                                const int at = nsrc + (j - base);
+                                W.srcp[at] = particle;
+    #pragma unroll
+                                for (int t = 0; t < T; ++t)
+                                    W.srcm[t][at] = reinterpret_cast<const uint32_t*>(W.pmask[t])[lo];
+                            }
+                            nsrc += window;
+                            base += window;
+                        }
                     }
                 }
                 __syncwarp();
@@ -823,8 +868,9 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
         if (nsrc > 0) flush_sources<H, T, kPot, kCount>(W, nsrc, lane, lane_bit, pos, G, X, e2, leaf_thr, A, WC);
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            if (!valid[t]) continue;
-            const int j = grp.start + lane + 32 * t;
+            const WalkGroup unit = groups[g];
+            if (lane + 32 * t >= unit.count) continue;
+            const int j = unit.start + lane + 32 * t;
             const int64_t i = fr.perm ? __ldg(fr.perm + j) : j;  // the target's particle
             const float4 a = make_float4(__fadd_rn(A[t].ax.x, A[t].ax.y), __fadd_rn(A[t].ay.x, A[t].ay.y),
                                          __fadd_rn(A[t].az.x, A[t].az.y), __fadd_rn(A[t].pot.x, A[t].pot.y));
@@ -1209,7 +1255,7 @@ walk_pair_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos, const 
                     : cls == kClassMixed
                         ? reinterpret_cast<const uint32_t*>(&W.half[rank & 1].nopen[rank >> 2])[(rank >> 1) & 1] : 0u;
                 int n_push = 0, n_src = 0;
-                if (my_open != 0u && code_b != kWalkSkipTag) {
+                if (my_open != 0u) {
                     if (code_b >= kWalkBucketTag) {
                         n_src = code_b - kWalkBucketTag;
                     } else {
@@ -1530,7 +1576,7 @@ frontier_kernel(Layout L, const float4* __restrict__ pos, const WalkNode* __rest
                 add_front += __popc(bm[h]);
                 n_push[h] = 0;
                 n_s[h] = 0;
-                if (cls[h] == kClassOpen && code_b[h] != kWalkSkipTag) {
+                if (cls[h] == kClassOpen) {
                     if (code_b[h] >= kWalkBucketTag) {
                         n_s[h] = code_b[h] - kWalkBucketTag;
                     } else {
