@@ -119,7 +119,7 @@ def build_ref(force: bool = False) -> dict:
     existing reference libraries are returned."""
     libs = {k: os.path.join(OUT, "lib%s.so" % k) for k in ("ref_cuda", "ref_cpu", "ref_morton")}
     libs["ic"] = build_ic(force)
-    if not os.path.isdir(REF):
+    if not os.path.isfile(os.path.join(REF, "cuda_engine.cu")):
         return {k: v for k, v in libs.items() if os.path.exists(v)}
     os.makedirs(BUILD, exist_ok=True)
     ref_srcs = [os.path.join(REF, f) for f in os.listdir(REF)]
