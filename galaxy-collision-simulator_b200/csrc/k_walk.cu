@@ -348,14 +348,14 @@ __device__ __forceinline__ void flush_sources(WarpSmem<H, T>& W, int nsrc, int l
     __syncwarp();
 }
 
-__device__ __forceinline__ uint32_t warp_exclusive_scan(uint32_t v, int lane) {
-    uint32_t x = v;
+// Sum of v over the lanes up to this one (a shuffle's own predicate says
+// whether it had a source lane).
+__device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, x, o);
-        if (lane >= o) x += y;
-    }
-    return x - v;
+    for (int o = 1; o < 32; o <<= 1)
+        asm volatile("{\n\t.reg .u32 r;\n\t.reg .pred p;\n\tshfl.sync.up.b32 r|p, %0, %1, 0, 0xffffffff;\n\t@p add.u32 %0, %0, r;\n\t}"
+            : "+r"(v) : "r"(o));
+    return v;
 }
 
 // A target's acceleration, and with an epilogue the step's kick/drift of its
@@ -737,8 +737,9 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                                                           : (2u << 16) - leaves * 0xFFFFu;
                     both += work[h];
                 }
-                const uint32_t excl = warp_exclusive_scan(both, lane);
-                const uint32_t total = __shfl_sync(kFull, excl + both, 31);
+                const uint32_t incl = warp_inclusive_scan(both);
+                const uint32_t excl = incl - both;
+                const uint32_t total = __shfl_sync(kFull, incl, 31);
                 {
                     int at = top + (int)(excl >> 16);
 #pragma unroll
@@ -1267,8 +1268,9 @@ walk_pair_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos, const 
                 W.cnt[w][lane] = own;
                 pair_sync(id);
                 const uint32_t other = W.cnt[w ^ 1][lane];
-                const uint32_t excl = warp_exclusive_scan(own + other, lane);
-                const uint32_t total = __shfl_sync(kFull, excl + own + other, 31);
+                const uint32_t incl = warp_inclusive_scan(own + other);
+                const uint32_t excl = incl - own - other;
+                const uint32_t total = __shfl_sync(kFull, incl, 31);
                 const uint32_t first = excl + (w ? other : 0u);  // this node's pushes and sources
                 if (n_push > 0) {
                     int at = top + (int)(first >> 16);
@@ -1588,8 +1590,9 @@ frontier_kernel(Layout L, const float4* __restrict__ pos, const WalkNode* __rest
                 lane_src += n_s[h];
             }
             const uint32_t both = ((uint32_t)lane_push << 16) | (uint32_t)lane_src;
-            const uint32_t excl = warp_exclusive_scan(both, lane);
-            const uint32_t total = __shfl_sync(kFull, excl + both, 31);
+            const uint32_t incl = warp_inclusive_scan(both);
+            const uint32_t excl = incl - both;
+            const uint32_t total = __shfl_sync(kFull, incl, 31);
             const int push_total = (int)(total >> 16), src_total = (int)(total & 0xFFFFu);
             if (n_take + n_front + add_take + add_front > kSuperCap || n_src + src_total > kSuperSrcCap ||
                 top + push_total > kFrontStack) {
