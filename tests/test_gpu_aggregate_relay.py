@@ -1,5 +1,6 @@
 """The aggregation above its blocks: sizes around the blocks' run of
-particles, segments that end inside and at the edge of a run, duplicate
+particles and the largest context one block takes whole (2,048), segments
+that end inside and at the edge of a run, duplicate
 positions (deep chains of equal keys), and an aggregation run again without a
 build.  Node masses, widths, boxes and centres of mass bit-exact against the
 oracle, segment by segment."""
@@ -27,7 +28,7 @@ def _stars(n, seed, dup):
 
 @pytest.mark.parametrize("dup", [0, 1])
 @pytest.mark.parametrize("com_fp64", [0, 1])
-@pytest.mark.parametrize("counts", [[2], [RUN - 1], [RUN], [RUN + 1], [2 * RUN], [1023], [1025], [20000],
+@pytest.mark.parametrize("counts", [[2], [RUN - 1], [RUN], [RUN + 1], [2 * RUN], [1023], [1025], [2048], [2049], [20000], [1200, 1, 847],
                                     [RUN, 1, RUN - 1, 2 * RUN, 3, 5000, 1]])
 def test_nodes_above_blocks(gcs_mod, oracle_mod, counts, com_fp64, dup):
     gcs = gcs_mod
