@@ -271,19 +271,20 @@ onesweep_kernel(Layout L, int shift, const uint64_t* __restrict__ keys_in,
     }
 }
 
+template <int kThreads, int... kItems>
+void configure_tiles() {
+    (cudaFuncSetAttribute(onesweep_kernel<kThreads, kItems, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)sizeof(SortSmem<kThreads, kItems, false>)), ...);
+    (cudaFuncSetAttribute(onesweep_kernel<kThreads, kItems, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)sizeof(SortSmem<kThreads, kItems, true>)), ...);
+}
+
 template <int kThreads, int kItems>
 void launch_tiles(const Layout& L, int pass, int tiles, const uint64_t* keys_in, const uint32_t* vals_in,
                   uint64_t* keys_out, uint32_t* vals_out, const uint32_t* hist, uint32_t* tile_counter,
                   uint32_t* lookback, uint32_t* status, cudaStream_t st) {
     constexpr size_t smem_key = sizeof(SortSmem<kThreads, kItems, false>);
     constexpr size_t smem_seg = sizeof(SortSmem<kThreads, kItems, true>);
-    static std::once_flag configured[kMaxDevices];
-    once_per_device(configured, [] {
-        cudaFuncSetAttribute(onesweep_kernel<kThreads, kItems, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_key);
-        cudaFuncSetAttribute(onesweep_kernel<kThreads, kItems, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_seg);
-    });
     if (pass < kKeyPasses) {
         launch_after(onesweep_kernel<kThreads, kItems, false>, (unsigned)tiles, kThreads, smem_key, st, L,
                      kRadixBits * pass, keys_in, vals_in, keys_out, vals_out, hist, tile_counter, lookback, status,
@@ -316,6 +317,13 @@ void launch_sort_pass(const Layout& L, int pass, const uint64_t* keys_in, const 
                       uint32_t* tile_counter, uint32_t* lookback, uint32_t* status,
                       cudaStream_t st) {
     if (L.n <= 0) return;
+    // every tile size at the first call on a device, so that a later call of
+    // another size may be its first within a stream capture
+    static std::once_flag configured[kMaxDevices];
+    once_per_device(configured, [] {
+        configure_tiles<256, kSortSmallTile / 256>();
+        configure_tiles<kSortThreads, 2, 3, 4, 5, 6, 7, kSortMaxItems>();
+    });
     const int tile = sort_tile(L.n);
     const int tiles = (L.n + tile - 1) / tile;
     uint32_t* lb = lookback + (size_t)pass * pass_words(L.n);
