@@ -1627,14 +1627,18 @@ int gcs_direct_accels_fp64(gcs_ctx* c, const gcs_params* p, int32_t segment,
             return GCS_ERR_NOMEM;
         c->targets_cap = n_targets;
     }
-    const int splits = direct_splits(n, n_targets);
+    int splits = direct_splits(n, n_targets);
     const size_t sums = splits > 1 ? 3 * (size_t)n_targets * (size_t)splits : 0;
     if (sums > c->direct_sums_cap) {
         if (c->direct_sums) cudaFree(c->direct_sums);
         c->direct_sums = nullptr;
         c->direct_sums_cap = 0;
-        if (dalloc(c, &c->direct_sums, sums)) return GCS_ERR_NOMEM;
-        c->direct_sums_cap = sums;
+        if (dalloc(c, &c->direct_sums, sums)) {
+            cudaGetLastError();
+            splits = 1;  // slower, but needs no work space
+        } else {
+            c->direct_sums_cap = sums;
+        }
     }
     GCS_CUDA(c, cudaMemcpyAsync(c->targets, targets, sizeof(int64_t) * (size_t)n_targets,
                                 cudaMemcpyHostToDevice, c->stream));

@@ -7,8 +7,11 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
+
+#include <unistd.h>
 
 namespace gcs {
 
@@ -46,6 +49,7 @@ struct HostCopy::Impl {
     std::condition_variable cv;
     std::atomic<bool> active{false};
     bool stop = false;
+    const pid_t owner = getpid();         // the process that has the helpers
     std::vector<std::thread> threads;
 
     bool copy_one() {
@@ -94,7 +98,8 @@ HostCopy* HostCopy::acquire() {
     if (!g_copy) {
         const int cores = (int)std::thread::hardware_concurrency();
         if (cores < 2) return nullptr;
-        Impl* im = new Impl();
+        Impl* im = new (std::nothrow) Impl();
+        if (!im) return nullptr;
         for (auto& d : im->done) d.store(0, std::memory_order_relaxed);
         if (cudaHostAlloc(reinterpret_cast<void**>(&im->ring), kPiece * kSlots, cudaHostAllocPortable) != cudaSuccess) {
             cudaGetLastError();
@@ -106,7 +111,11 @@ HostCopy* HostCopy::acquire() {
             for (int k = 0; k < std::min(kWorkers, cores - 1); ++k) im->threads.emplace_back([im] { im->help(); });
         } catch (...) {  // fewer threads, or none: the caller's own still copies
         }
-        g_copy = new HostCopy();
+        g_copy = new (std::nothrow) HostCopy();
+        if (!g_copy) {
+            delete im;
+            return nullptr;
+        }
         g_copy->impl = im;
     }
     ++g_users;
@@ -122,7 +131,9 @@ void HostCopy::release() {
             g_copy = nullptr;
         }
     }
-    delete last;
+    // a forked child has the object but not its threads: joining them would
+    // wait for good, so there it is left to the end of the process
+    if (last && last->impl->owner == getpid()) delete last;
 }
 
 bool HostCopy::begin() {
