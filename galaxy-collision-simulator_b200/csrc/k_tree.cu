@@ -273,7 +273,8 @@ struct AggSmem {
     int32_t arrived[kRange];
     uint16_t queue[3][kRange / 2 + 1];  // nodes whose children are both finished, by step
     int n_queue[3];
-    int n_roots;                  // finished subtrees whose parent lies above the block
+    int32_t root[kRange == kAggRange ? kRange : 1];  // finished subtree whose parent lies above the block, at
+                                                     // its first particle (-1: none starts here)
 };
 constexpr int kNotLocal = -2;
 constexpr int kAggWholeMax = 2048;   // particles one block takes whole
@@ -314,8 +315,9 @@ __device__ __forceinline__ ChildData smem_node(const AggSmem<kRange>& S, int slo
 //           step computes the nodes whose two children are finished, packed
 //           into whole warps (a step waits on no global load, store or
 //           fence, and a climb by every particle's own lane keeps 8 lanes of
-//           a warp busy).  A subtree whose parent is not local is left on a
-//           list;
+//           a warp busy).  A subtree whose parent is not local is marked at
+//           its first particle;
+//   list    the marked subtrees, by position (rise_kernel relies on it);
 //   store   the finished nodes' records, whole and coalesced.
 // The nodes above the blocks are rise_kernel's.
 // A context of up to kAggWholeMax particles is one block's run: no node is
@@ -331,10 +333,9 @@ aggregate_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __re
     AggSmem<kRange>& S = *reinterpret_cast<AggSmem<kRange>*>(agg_smem);
     const int ni = L.n_internal;
     const int lim = ni + L.n;
-    if (threadIdx.x == 0) {
-        S.n_roots = 0;
-        S.n_queue[0] = S.n_queue[1] = S.n_queue[2] = 0;
-    }
+    if (threadIdx.x == 0) S.n_queue[0] = S.n_queue[1] = S.n_queue[2] = 0;
+    if (!kWhole)
+        for (int j = threadIdx.x; j < kRange; j += kThreads) S.root[j] = -1;
     const int b0 = blockIdx.x * kRange;
     const int count = min(kRange, L.n - b0);
     let_next_start();
@@ -368,13 +369,14 @@ aggregate_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __re
     __syncthreads();
 
     // ---- climb
-    // arrive: `from` is finished; the second child to arrive at a local parent
-    // queues it for the next step, a subtree under any other parent is a root
-    const auto arrive = [&](int from, int up, int sg, int q) {
+    // arrive: `from` (its first particle in slot `first`) is finished; the
+    // second child to arrive at a local parent queues it for the next step, a
+    // subtree under any other parent is a root
+    const auto arrive = [&](int from, int first, int up, int sg, int q) {
         if (up < 0) return;  // the segment's root (or a one-particle segment)
         const int slot = up + sg - b0;
         if (slot < 0 || slot >= count || S.link[slot].w == kNotLocal) {
-            roots[b0 + atomicAdd(&S.n_roots, 1)] = make_int2(from, sg);
+            if (!kWhole) S.root[first] = from;
         } else if (atomicAdd(&S.arrived[slot], 1) == 1) {
             S.queue[q][atomicAdd(&S.n_queue[q], 1)] = (uint16_t)slot;
         }
@@ -382,7 +384,7 @@ aggregate_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __re
 #pragma unroll
     for (int u = 0; u < kRange / kThreads; ++u) {
         const int j = threadIdx.x + u * kThreads;
-        if (j < count) arrive(ni + b0 + j, my_parent[u], seg_of(b0 + j), 0);
+        if (j < count) arrive(ni + b0 + j, j, my_parent[u], seg_of(b0 + j), 0);
     }
     __syncthreads();
     for (int step = 0; S.n_queue[step % 3] > 0; ++step) {
@@ -430,9 +432,24 @@ aggregate_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __re
             S.com_m[slot] = make_float4(node.com.x, node.com.y, node.com.z, node.m);
             S.box_a[slot] = make_float4(node.lo.x, node.lo.y, node.lo.z, node.hi.x);
             S.box_b[slot] = make_float2(node.hi.y, node.hi.z);
-            arrive(b0 + slot - sg, k.w, sg, (step + 1) % 3);
+            arrive(b0 + slot - sg, min(b0 + slot, k.z) - b0, k.w, sg, (step + 1) % 3);
         }
         __syncthreads();
+    }
+
+    // ---- list
+    if (!kWhole && threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int listed = 0;
+#pragma unroll
+        for (int j0 = 0; j0 < kRange; j0 += 32) {
+            const int from = S.root[j0 + lane];
+            const uint32_t marked = __ballot_sync(0xFFFFFFFFu, from >= 0);
+            if (from >= 0)
+                roots[b0 + listed + __popc(marked & ((1u << lane) - 1u))] = make_int2(from, seg_of(b0 + j0 + lane));
+            listed += __popc(marked);
+        }
+        if (lane == 0) n_roots[blockIdx.x] = (uint32_t)listed;
     }
 
     // ---- store
@@ -452,17 +469,23 @@ aggregate_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __re
         write_walk_node(wnp, node, make_float3(c.x, c.y, c.z), c.w, width, k.x, k.y, g, k.z,
                             L.nseg > 1 ? (int)__ldg(L.seg_off + s) : 0, seg_end(s) - 1, ni);
     }
-    __syncthreads();
-
-    if (!kWhole && threadIdx.x == 0) n_roots[blockIdx.x] = (uint32_t)S.n_roots;
 }
 
-// Climbs on from the subtrees the blocks' climbs left (one warp for each
-// run of kRange particles, one lane for each of its subtrees): a left child
-// hands its values to the relay and stops, a right child waits for the left
-// one's, computes the node and goes on.  The left child's particles, and so
-// its climber, come first, and blocks take their runs in launch order from a
-// ticket: whoever is waited for is running or done.  The wait is bounded.
+// Climbs on from the subtrees the blocks' climbs left, one warp for each run
+// of kAggRange particles: lane l takes the subtrees l, l + 32, ... of the run's
+// list one after another (a run has one subtree per level of the paths at its
+// two ends: up to 18 in a smooth collision, above 60 in a steep profile).  A
+// left child hands its values to the relay and stops, a right child waits for
+// the left one's, computes the node and goes on.
+//
+// No wait is for something that has not started.  A climber waits only for a
+// left sibling of its own subtree, and that sibling's values come from a
+// climber that started at a lower position.  Lists are in the order of
+// position, so within a run that climber is an earlier entry: in the same turn
+// of the warp, on another lane, or in a turn that is over.  Between runs it is
+// one of an earlier run, and blocks take their runs in launch order from a
+// ticket.  So the lowest waiting climber can always go on.  The wait is
+// bounded all the same.
 // A node above the blocks: its links, and which of it and its children are
 // FP64 nodes.
 struct RiseNode {
@@ -558,12 +581,8 @@ rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restric
     const int lim = ni + L.n;
     const int count = min((int)__ldg(n_roots + run), kAggRange);
     const bool fp64 = com_fp64 != 0;
-    for (int r = lane; r < count; r += 32) {
-        // the finished subtree `from`, its values, and its parent
-        const int2 root = roots[run * kAggRange + r];
-        int from = root.x;
-        const int s = root.y;
-        ChildData mine;
+    // the finished subtree `from`: its values, and the node above it
+    const auto start = [&](int from, int s, ChildData& mine) {
         int node;
         if (from >= ni) {
             const float4 p = __ldg(pos + (from - ni));
@@ -582,12 +601,25 @@ rise_kernel(Layout L, const float4* __restrict__ pos, BvhNodeTraverse* __restric
         }
         mine.mx = make_double3(0.0, 0.0, 0.0);
         mine.md = 0.0;
+        return rise_node(tr, bd, node, s, ni, fp64);
+    };
+    // left children of the later turns hand over before any wait of the first
+    for (int r = lane + 32; r < count; r += 32) {
+        const int2 root = roots[run * kAggRange + r];
+        ChildData mine;
+        const RiseNode N = start(root.x, root.y, mine);
+        if (N.node >= 0 && valid_links(N, root.x, lim) && N.cl == root.x) hand_over(wnp.wn, tr, bd, com64, N, mine);
+    }
+    for (int r = lane; r < count; r += 32) {
+        const int2 root = roots[run * kAggRange + r];
+        const int s = root.y;
+        ChildData mine;
+        RiseNode N = start(root.x, s, mine);
         const int seg_lo = L.nseg > 1 ? (int)__ldg(L.seg_off + s) : 0;
         const int seg_hi = (L.nseg > 1 ? (int)__ldg(L.seg_off + s + 1) : L.n) - 1;
-        RiseNode N = rise_node(tr, bd, node, s, ni, fp64);
-        bool ok = N.node >= 0 && valid_links(N, from, lim);
-        if (ok && N.cl == from) {
-            hand_over(wnp.wn, tr, bd, com64, N, mine);
+        bool ok = N.node >= 0 && valid_links(N, root.x, lim);
+        if (ok && N.cl == root.x) {
+            if (r < 32) hand_over(wnp.wn, tr, bd, com64, N, mine);
             continue;
         }
         RelayWords w;
