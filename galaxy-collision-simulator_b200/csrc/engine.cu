@@ -50,6 +50,7 @@ struct gcs_ctx {
     int sorted_buf = 0;
     bool scratch_zeroed = false;  // within run_stages: the accumulated scratch is already zero
     bool front = false;  // small scenarios sort in one launch (k_front.cu)
+    bool hist_counted = true;  // the digit histograms are those of keys[0] (not after that launch)
     BvhNodeTraverse* tr = nullptr;
     BvhNodeBuild* bd = nullptr;
     // Walk records (one per internal node) and what they were written for:
@@ -531,9 +532,15 @@ static int run_stage(gcs_ctx* c, const gcs_params* p, int stage, bool gather_bes
                 GCS_CUDA(c, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kRadix * (size_t)passes, st));
             launch_encode(L, c->pos[c->cur], p->bounds_mode, p->global_min, p->global_max,
                           c->seg_bounds, c->keys[0], c->idx[0], hist, seg_passes(c->nseg), st);
+            c->hist_counted = true;
             return check_launch(c, "encode");
         case GCS_STAGE_SORT: {
             if (!c->scratch_zeroed) GCS_CUDA(c, cudaMemsetAsync(c->scratch + sl.tiles, 0, sl.end - sl.tiles, st));
+            if (!c->hist_counted) {  // the sort run again on what the one launch sorted
+                GCS_CUDA(c, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kRadix * kKeyPasses, st));
+                launch_key_histograms(c->keys[0], c->n, hist, st);
+                c->hist_counted = true;
+            }
             for (int pass = 0; pass < passes; ++pass) {
                 const int in = pass & 1;
                 launch_sort_pass(L, pass, c->keys[in], c->idx[in], c->keys[in ^ 1], c->idx[in ^ 1],
@@ -611,6 +618,9 @@ static int run_stage(gcs_ctx* c, const gcs_params* p, int stage, bool gather_bes
     }
 }
 
+// Whether bounds, encode and sort, run in one call, are one launch.
+static bool one_launch_sort(const gcs_ctx* c) { return c->nseg == 1 && c->n <= kFrontMax && c->front; }
+
 static int run_stages(gcs_ctx* c, const gcs_params* p, int first, int last) {
     if (!c) return GCS_ERR_ARG;
     int rc = validate_params(c, p);
@@ -626,11 +636,12 @@ static int run_stages(gcs_ctx* c, const gcs_params* p, int first, int last) {
     const bool gather_beside_build = first <= GCS_STAGE_GATHER && last >= GCS_STAGE_BUILD;
     const bool kick_in_walk = first <= GCS_STAGE_WALK && last >= GCS_STAGE_INTEGRATE && c->range_count < 0;
     int s = first;
-    if (first <= GCS_STAGE_ENCODE && last >= GCS_STAGE_SORT && c->nseg == 1 && c->n <= kFrontMax && c->front) {
+    if (first <= GCS_STAGE_ENCODE && last >= GCS_STAGE_SORT && one_launch_sort(c)) {
         // a small scenario: bounds, encode and sort in one launch
         const int bounds = p->bounds_mode != GCS_BOUNDS_DEVICE ? kFrontBoundsCaller
                          : first == GCS_STAGE_BOUNDS ? kFrontBoundsReduce : kFrontBoundsGiven;
         c->sorted_buf = 0;  // as after kKeyPasses passes
+        c->hist_counted = false;
         launch_front(c->pos[c->cur], c->n, bounds, p->global_min, p->global_max, c->seg_bounds, c->keys[0], c->idx[0],
                      c->status, c->stream);
         rc = check_launch(c, "bounds, encode and sort");
@@ -1131,6 +1142,7 @@ int gcs_step(gcs_ctx* c, const gcs_params* p) {
     GCS_CUDA(c, cudaGraphLaunch(c->graph_exec[c->cur], c->stream));
     c->cur = c->graph_after[c->cur];  // the flips the captured step made (gather, kick/drift in the walk)
     c->sorted_buf = (kKeyPasses + seg_passes(c->nseg)) & 1;
+    c->hist_counted = !one_launch_sort(c);
     c->relay_empty = false;  // the captured aggregation used it
     return GCS_OK;
 }

@@ -138,6 +138,9 @@ bool front_available();
 void launch_front(const float4* pos, int n, int front_bounds, float gmin, float gmax, float2* seg_bounds,
                   uint64_t* keys, uint32_t* idx, uint32_t* status, cudaStream_t st);
 
+// Digit histograms of the keys' kKeyPasses digits, added to hist
+// (sort_static.cu; encode counts its own).
+void launch_key_histograms(const uint64_t* keys, int64_t n, uint32_t* hist, cudaStream_t st);
 size_t sort_lookback_words(int64_t n, int passes);
 size_t sort_lookback_words_upto(int64_t n, int passes);  // the most any m <= n needs
 void launch_sort_pass(const Layout& L, int pass, const uint64_t* keys_in, const uint32_t* vals_in,

@@ -106,6 +106,11 @@ int scratch_address(uint32_t** out) {
 }
 
 }  // namespace
+
+void launch_key_histograms(const uint64_t* keys, int64_t n, uint32_t* hist, cudaStream_t st) {
+    launch_after(key_histograms_kernel, count_grid(n, current_sm_count()), kCountThreads, 0, st, keys, n, hist);
+}
+
 }  // namespace gcs
 
 extern "C" int gcs_sort_pairs_static(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt,
@@ -129,7 +134,7 @@ extern "C" int gcs_sort_pairs_static(uint64_t* keys, uint32_t* vals, uint64_t* k
     uint32_t* lookback = own_status + kStatusWords;
     const size_t clear_words = kHistWords + kTicketWords + kStatusWords + sort_lookback_words(n, kKeyPasses);
     if (cudaMemsetAsync(base, 0, clear_words * sizeof(uint32_t), st) != cudaSuccess) return GCS_ERR_CUDA;
-    launch_after(key_histograms_kernel, count_grid(n, current_sm_count()), kCountThreads, 0, st, keys, n, hist);
+    launch_key_histograms(keys, n, hist, st);
     Layout L;
     L.n = (int32_t)n;
     L.nseg = 1;
