@@ -577,12 +577,15 @@ static int run_stage(gcs_ctx* c, const gcs_params* p, int stage, bool gather_bes
             return check_launch(c, "build");
         case GCS_STAGE_AGGREGATE: {
             const WalkNodeParams wnp = walk_node_params(c, p);
+            // its lists of subtrees stand where the walk stage's frontier lists
+            // will (kSuperCap words for at most kSuperTargets particles)
+            int2* roots = reinterpret_cast<int2*>(c->sg_list);
+            uint32_t* n_roots = reinterpret_cast<uint32_t*>(roots + c->capacity);
             uint32_t* ticket = scratch_at<uint32_t>(c, sl.agg_q);
             if (!c->relay_empty) launch_relay_reset(L, c->tr, c->bd, c->wn, c->com64, ticket, st);
             c->relay_empty = false;
             launch_aggregate(L, c->pos[c->cur], c->tr, c->bd, c->com64, c->leaf_parent, p->com_fp64, wnp,
-                             reinterpret_cast<int2*>(c->keys[c->sorted_buf ^ 1]), c->idx[c->sorted_buf ^ 1], ticket,
-                             c->status, st);
+                             roots, n_roots, ticket, c->status, st);
             c->tree_gen++;
             c->wn_gen = c->tree_gen;
             c->wn_G = wnp.G;
@@ -811,6 +814,7 @@ static int allocate_state(gcs_ctx* c) {
     const size_t max_supers = N / (size_t)(kSuperTargets - kGroupSize) + (size_t)max_segments + 1;
     c->supers_cap = max_supers;
     if (!rc) rc |= dalloc(c, &c->supers, max_supers);
+    static_assert(kSuperCap / kSuperTargets >= 3, "the aggregation's lists fit sg_list: 3 words a particle");
     if (!rc) rc |= dalloc(c, &c->sg_list, max_supers * (size_t)kSuperCap);
     if (!rc) rc |= dalloc(c, &c->sg_src, max_supers * (size_t)kSuperSrcCap);
     if (!rc) rc |= dalloc(c, &c->sg_meta, max_supers);

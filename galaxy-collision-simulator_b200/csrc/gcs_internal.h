@@ -156,7 +156,8 @@ struct WalkNodeParams;
 // tr, bd and com64 of the nodes above its blocks) and zeroes its block ticket; an
 // aggregation that does not follow a build needs launch_relay_reset first.
 // roots, n_roots: the aggregation's lists between its two launches, n records
-// each (the sort's spare key and index buffers).
+// and a word a run (not the sort's spare buffers: with an odd number of passes
+// those hold the pairs that a sort stage run again would start from).
 void launch_build(const Layout& L, const uint64_t* keys, BvhNodeTraverse* tr, BvhNodeBuild* bd,
                   int32_t* leaf_parent, WalkNode* wn, double4* com64, uint32_t* agg_ticket, uint32_t* status,
                   cudaStream_t st);

@@ -38,6 +38,18 @@ def test_one_segment(gcs_mod, n, last):
         _same_again(gcs, ctx, p)
 
 
+@pytest.mark.parametrize("last", ["SORT", "BUILD", "AGGREGATE", "INTEGRATE"])
+@pytest.mark.parametrize("counts", [[1, 700, 5000], [1000] * 3 + [1] * 300, [30000, 40000]])
+def test_segments(gcs_mod, counts, last):
+    gcs = gcs_mod
+    p = gcs.reference_params(bounds_mode=gcs.BOUNDS_DEVICE)
+    with gcs.Context(sum(counts), len(counts)) as ctx:
+        ctx.set_segments(counts)
+        ctx.upload(_stars(sum(counts), 7))
+        ctx.run_stages(p, gcs.STAGE_BOUNDS, getattr(gcs, "STAGE_" + last))
+        _same_again(gcs, ctx, p)
+
+
 def test_after_a_captured_step(gcs_mod):
     import torch
     gcs = gcs_mod
