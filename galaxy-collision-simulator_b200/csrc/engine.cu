@@ -1146,8 +1146,13 @@ int gcs_step(gcs_ctx* c, const gcs_params* p) {
     GCS_CUDA(c, cudaGraphLaunch(c->graph_exec[c->cur], c->stream));
     c->cur = c->graph_after[c->cur];  // the flips the captured step made (gather, kick/drift in the walk)
     c->sorted_buf = (kKeyPasses + seg_passes(c->nseg)) & 1;
+    // what the captured stages leave behind
     c->hist_counted = !one_launch_sort(c);
-    c->relay_empty = false;  // the captured aggregation used it
+    c->relay_empty = false;
+    const WalkNodeParams wnp = walk_node_params(c, p);
+    c->wn_gen = ++c->tree_gen;
+    c->wn_G = wnp.G;
+    c->wn_L = wnp.leaf_size;
     return GCS_OK;
 }
 
