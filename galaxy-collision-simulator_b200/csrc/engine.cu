@@ -1667,9 +1667,25 @@ int gcs_direct_accels_fp64(gcs_ctx* c, const gcs_params* p, int32_t segment,
                        (double)p->epsilon_sq, c->direct_sums, c->direct_out, c->stream);
     int rc = check_launch(c, "direct_fp64");
     if (rc) return rc;
-    GCS_CUDA(c, cudaMemcpyAsync(out, c->direct_out, sizeof(double) * 3 * (size_t)n_targets,
-                                cudaMemcpyDeviceToHost, c->stream));
-    GCS_CUDA(c, cudaStreamSynchronize(c->stream));
+    const auto read_back = [&] {
+        const cudaError_t e = cudaMemcpyAsync(out, c->direct_out, sizeof(double) * 3 * (size_t)n_targets,
+                                              cudaMemcpyDeviceToHost, c->stream);
+        return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+    };
+    GCS_CUDA(c, read_back());
+    // a NaN among them makes their sum one (in eight parts, for its latency)
+    double part[8] = {};
+    int64_t i = 0;
+    for (; i + 8 <= 3 * n_targets; i += 8)
+        for (int k = 0; k < 8; ++k) part[k] += out[i + k];
+    for (; i < 3 * n_targets; ++i) part[0] += out[i];
+    const double all = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
+    if (all == all) return GCS_OK;
+    launch_direct_nonfinite(c->pos[c->cur], first, n, c->targets, n_targets, (double)p->G, (double)p->epsilon_sq,
+                            c->direct_out, c->stream);
+    rc = check_launch(c, "direct_fp64");
+    if (rc) return rc;
+    GCS_CUDA(c, read_back());
     return GCS_OK;
 }
 

@@ -328,5 +328,8 @@ int direct_splits(int64_t seg_n, int64_t n_targets);
 void launch_direct_fp64(const float4* pos, int64_t seg_first, int64_t seg_n, const int64_t* targets,
                         int64_t n_targets, int splits, double G, double eps2, double* sums, double* out,
                         cudaStream_t st);
+// The targets whose sums in out hold a NaN again, as sums over any input give.
+void launch_direct_nonfinite(const float4* pos, int64_t seg_first, int64_t seg_n, const int64_t* targets,
+                             int64_t n_targets, double G, double eps2, double* out, cudaStream_t st);
 
 }  // namespace gcs

@@ -295,9 +295,8 @@ __global__ void diag_kernel(const float4* __restrict__ pos, const float4* __rest
 // g x^(-3/2) to double precision: the hardware estimate y of x^(-1/2), with
 // e = 1 - x y^2, and the first terms of the binomial series
 // x^(-3/2) = y^3 (1 - e)^(-3/2) = y^3 (1 + 3/2 e + 15/8 e^2 + ...).  The
-// estimate is good to about 2^-20, which leaves a term below 2^-55.  x = 0 and
-// infinity give NaN, which the direct sum's terms are there in any case (0
-// times infinity).
+// estimate is good to about 2^-20, which leaves a term below 2^-55.  An
+// infinite or zero x and an infinite g give NaN (direct_nonfinite_kernel).
 __device__ __forceinline__ double times_inv_r3(double g, double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -387,6 +386,47 @@ direct_fp64_kernel(const float4* __restrict__ pos, int64_t seg_first, int64_t se
         double x = 0;
         for (int w = 0; w < kDirectThreads / 32; ++w) x += s[threadIdx.x][w];
         sums[3 * (n_targets * blockIdx.y + first) + threadIdx.x] = x;
+    }
+}
+
+// Sums with a NaN component again, a block per target, term by term as written
+// down: a source infinitely far away adds NaN to the components in which it is
+// and nothing to the others, where times_inv_r3 makes all three NaN.  Launched
+// only where the caller has seen a NaN (the choice made inside
+// direct_fp64_kernel, by pair, by source or after its loop: 1,545 us in place
+// of 1,395).
+__global__ void __launch_bounds__(kStreamThreads)
+direct_nonfinite_kernel(const float4* __restrict__ pos, int64_t seg_first, int64_t seg_n,
+                        const int64_t* __restrict__ targets, int64_t n_targets, double G, double eps2,
+                        double* __restrict__ out) {
+    __shared__ double s[3][kStreamThreads / 32];
+    for (int64_t t = blockIdx.x; t < n_targets; t += gridDim.x) {
+        if (!isnan(out[3 * t]) && !isnan(out[3 * t + 1]) && !isnan(out[3 * t + 2])) continue;  // the same in all threads
+        const int64_t ti = __ldg(targets + t);
+        const float4 q = __ldg(pos + seg_first + ti);
+        double a[3] = {0.0, 0.0, 0.0};
+        for (int64_t j = threadIdx.x; j < seg_n; j += kStreamThreads) {
+            if (j == ti) continue;
+            const float4 p = __ldg(pos + seg_first + j);
+            const double dx = (double)p.x - q.x, dy = (double)p.y - q.y, dz = (double)p.z - q.z;
+            const double inv = 1.0 / sqrt(dx * dx + dy * dy + dz * dz + eps2);
+            const double f = G * (double)p.w * inv * inv * inv;
+            a[0] += f * dx;
+            a[1] += f * dy;
+            a[2] += f * dz;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            for (int o = 16; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xFFFFFFFFu, a[k], o);
+            if ((threadIdx.x & 31) == 0) s[k][threadIdx.x >> 5] = a[k];
+        }
+        __syncthreads();  // (also: every thread has read out)
+        if (threadIdx.x < 3) {
+            double x = 0.0;
+            for (int w = 0; w < kStreamThreads / 32; ++w) x += s[threadIdx.x][w];
+            out[3 * t + threadIdx.x] = x;
+        }
+        __syncthreads();
     }
 }
 
@@ -487,6 +527,13 @@ void launch_direct_fp64(const float4* pos, int64_t seg_first, int64_t seg_n, con
                                                         (seg_n + splits - 1) / splits, G, eps2, to);
     if (splits > 1)
         direct_sum_kernel<<<(unsigned)((3 * n_targets + 255) / 256), 256, 0, st>>>(sums, splits, 3 * n_targets, out);
+}
+
+void launch_direct_nonfinite(const float4* pos, int64_t seg_first, int64_t seg_n, const int64_t* targets,
+                             int64_t n_targets, double G, double eps2, double* out, cudaStream_t st) {
+    const int64_t cap = (int64_t)current_sm_count() * 16;
+    direct_nonfinite_kernel<<<(unsigned)std::min(n_targets, cap), kStreamThreads, 0, st>>>(pos, seg_first, seg_n, targets,
+                                                                                         n_targets, G, eps2, out);
 }
 
 }  // namespace gcs
