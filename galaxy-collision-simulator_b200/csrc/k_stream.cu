@@ -307,7 +307,7 @@ __device__ __forceinline__ double times_inv_r3(double g, double x) {
 }
 
 // FP64 direct sum, excluding only the target itself: a block takes
-// kDirectTargets targets (held in registers, with their sums) and every
+// kTargets targets (held in registers, with their sums) and every
 // kDirectThreads-th source of its split of the segment; the splits' sums are
 // added in order by direct_sum_kernel.  Only sources between the block's
 // first and last target can be one of its targets; the others are summed
@@ -318,21 +318,27 @@ __device__ __forceinline__ double times_inv_r3(double g, double x) {
 // every pair, needed about three times as many).  4,096 targets of 262,144
 // particles: 2.86 ms before, 1.41 ms now (800 G pairs/s at 65,536
 // targets, 69 % of the pipe at 1,965 MHz); 3, 6 and 8 targets a block 1.46, 1.35
-// and 2.1 ms, 6 slower where targets are few.
+// and 2.1 ms, 6 slower where targets are few.  Up to eight targets an SM the
+// chip is not full and a call takes as long as a block: two a block then
+// (16 targets of 1,000 particles, whole call: 35.5 us with four, 28.9 with two,
+// 30.5 with the earlier kernel; 1,000 of 262,144: 403 and 394; 4,000 of 30,000:
+// 213 and 224).
 constexpr int kDirectThreads = 128;
 constexpr int kDirectTargets = 4;
+constexpr int kDirectFewTargets = 2;
 
+template <int kTargets>
 __global__ void __launch_bounds__(kDirectThreads)
 direct_fp64_kernel(const float4* __restrict__ pos, int64_t seg_first, int64_t seg_n,
                    const int64_t* __restrict__ targets, int64_t n_targets, int64_t per_split, double G, double eps2,
                    double* __restrict__ sums) {
-    double tx[kDirectTargets], ty[kDirectTargets], tz[kDirectTargets];
-    double ax[kDirectTargets] = {}, ay[kDirectTargets] = {}, az[kDirectTargets] = {};
-    const int64_t first = (int64_t)blockIdx.x * kDirectTargets;
+    double tx[kTargets], ty[kTargets], tz[kTargets];
+    double ax[kTargets] = {}, ay[kTargets] = {}, az[kTargets] = {};
+    const int64_t first = (int64_t)blockIdx.x * kTargets;
     const auto target = [&](int t) { return __ldg(targets + (first + t < n_targets ? first + t : n_targets - 1)); };
     int64_t t_min = seg_n, t_max = -1;
 #pragma unroll
-    for (int t = 0; t < kDirectTargets; ++t) {
+    for (int t = 0; t < kTargets; ++t) {
         const int64_t ti = target(t);
         t_min = ti < t_min ? ti : t_min;
         t_max = ti > t_max ? ti : t_max;
@@ -347,7 +353,7 @@ direct_fp64_kernel(const float4* __restrict__ pos, int64_t seg_first, int64_t se
         const double sx = p.x, sy = p.y, sz = p.z, gm = G * (double)p.w;
         if (j < t_min || j > t_max) {
 #pragma unroll
-            for (int t = 0; t < kDirectTargets; ++t) {
+            for (int t = 0; t < kTargets; ++t) {
                 const double dx = sx - tx[t], dy = sy - ty[t], dz = sz - tz[t];
                 const double f = times_inv_r3(gm, fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
                 ax[t] = fma(f, dx, ax[t]);
@@ -356,7 +362,7 @@ direct_fp64_kernel(const float4* __restrict__ pos, int64_t seg_first, int64_t se
             }
         } else {
 #pragma unroll
-            for (int t = 0; t < kDirectTargets; ++t) {
+            for (int t = 0; t < kTargets; ++t) {
                 const double dx = sx - tx[t], dy = sy - ty[t], dz = sz - tz[t];
                 const double f = times_inv_r3(gm, fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
                 if (j != target(t)) {
@@ -367,9 +373,9 @@ direct_fp64_kernel(const float4* __restrict__ pos, int64_t seg_first, int64_t se
             }
         }
     }
-    __shared__ double s[3 * kDirectTargets][kDirectThreads / 32];
+    __shared__ double s[3 * kTargets][kDirectThreads / 32];
 #pragma unroll
-    for (int t = 0; t < kDirectTargets; ++t) {
+    for (int t = 0; t < kTargets; ++t) {
         for (int o = 16; o > 0; o >>= 1) {
             ax[t] += __shfl_xor_sync(0xFFFFFFFFu, ax[t], o);
             ay[t] += __shfl_xor_sync(0xFFFFFFFFu, ay[t], o);
@@ -382,7 +388,7 @@ direct_fp64_kernel(const float4* __restrict__ pos, int64_t seg_first, int64_t se
         }
     }
     __syncthreads();
-    if (threadIdx.x < 3 * kDirectTargets && first + threadIdx.x / 3 < n_targets) {
+    if (threadIdx.x < 3 * kTargets && first + threadIdx.x / 3 < n_targets) {
         double x = 0;
         for (int w = 0; w < kDirectThreads / 32; ++w) x += s[threadIdx.x][w];
         sums[3 * (n_targets * blockIdx.y + first) + threadIdx.x] = x;
@@ -521,10 +527,15 @@ void launch_direct_fp64(const float4* pos, int64_t seg_first, int64_t seg_n, con
                         int64_t n_targets, int splits, double G, double eps2, double* sums, double* out,
                         cudaStream_t st) {
     if (n_targets <= 0) return;
-    const dim3 grid((unsigned)((n_targets + kDirectTargets - 1) / kDirectTargets), (unsigned)splits);
     double* to = splits > 1 ? sums : out;
-    direct_fp64_kernel<<<grid, kDirectThreads, 0, st>>>(pos, seg_first, seg_n, targets, n_targets,
-                                                        (seg_n + splits - 1) / splits, G, eps2, to);
+    const int64_t per_split = (seg_n + splits - 1) / splits;
+    const auto blocks = [&](int per) { return dim3((unsigned)((n_targets + per - 1) / per), (unsigned)splits); };
+    if (n_targets <= (int64_t)current_sm_count() * 8)
+        direct_fp64_kernel<kDirectFewTargets><<<blocks(kDirectFewTargets), kDirectThreads, 0, st>>>(
+            pos, seg_first, seg_n, targets, n_targets, per_split, G, eps2, to);
+    else
+        direct_fp64_kernel<kDirectTargets><<<blocks(kDirectTargets), kDirectThreads, 0, st>>>(
+            pos, seg_first, seg_n, targets, n_targets, per_split, G, eps2, to);
     if (splits > 1)
         direct_sum_kernel<<<(unsigned)((3 * n_targets + 255) / 256), 256, 0, st>>>(sums, splits, 3 * n_targets, out);
 }
