@@ -295,6 +295,19 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
                  int sm_count, unsigned long long* counts, int2* gstack, size_t gstack_entries,
                  cudaStream_t st, const WalkEpilogue& ep = WalkEpilogue(),
                  const WalkFrontier& fr = WalkFrontier());
+// Whether every group gets two warps: while all groups find a pair of warps
+// within two waves.  Walk stage in us, one warp a group / two (theta 0.5, leaf
+// 8, batch 64 from 16,384 on):
+//    1,408 particles  78 /  61       60,000 (0.7, leaf 4)     170 / 139
+//    8,192           170 / 121       75,000                   326 / 285
+//   16,384           199 / 135       110,000                  406 / 385
+//   45,056           309 / 225       131,072 (0.7, leaf 4)    289 / 295
+//   16 x 5,000       170 / 152       262,144                  737 / 770
+// A caller's walk_blocks_per_sm is an occupancy of the one-warp kernel, so
+// setting it asks for that one.
+inline bool walk_pairs_pay(int n_groups, int sm_count, int blocks_per_sm) {
+    return blocks_per_sm <= 0 && n_groups <= 20 * sm_count;
+}
 int walk_max_blocks_per_sm(int batch, int with_potential, int targets_per_lane);
 // Persistent walk grid (blocks) for n_groups groups, and the global stack
 // entries that grid needs.

@@ -1734,16 +1734,6 @@ static void launch_ht(const Layout& L, const WalkParams& q, const float4* pos, c
     }
 }
 
-// Whether every group gets two warps: while all groups find a pair of warps
-// within two waves.  Walk stage in us, one warp a group / two (theta 0.5, leaf
-// 8, batch 64 from 16,384 on):
-//    1,408 particles  78 /  61       60,000 (0.7, leaf 4)     170 / 139
-//    8,192           170 / 121       75,000                   326 / 285
-//   16,384           199 / 135       110,000                  406 / 385
-//   45,056           309 / 225       131,072 (0.7, leaf 4)    289 / 295
-//   16 x 5,000       170 / 152       262,144                  737 / 770
-static bool pairs_pay(int n_groups, int sm_count) { return n_groups <= 20 * sm_count; }
-
 template <int H>
 static void launch_pairs(const Layout& L, const WalkParams& q, const float4* pos, const WalkNode* wn,
                          const WalkGroup* groups, int n_groups, float4* acc, uint32_t* queue, uint32_t* status,
@@ -1813,7 +1803,7 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
     // entries per warp region: the whole buffer split over this grid's warps
     const size_t units = gstack_entries / ((size_t)grid * kWalkWarps);
     const int cap = (int)(std::min<size_t>(units, (size_t)1 << 24) / (size_t)T);
-    if (T == 1 && !counts && pairs_pay(n_groups, sm_count)) {
+    if (T == 1 && !counts && walk_pairs_pay(n_groups, sm_count, blocks_per_sm)) {
         // two warps a group; the stack regions are shared out over the pairs
         const int64_t blocks = ((int64_t)n_groups + kPairBlockPairs - 1) / kPairBlockPairs;
         const int64_t pairs = blocks * kPairBlockPairs;

@@ -69,7 +69,9 @@ typedef struct gcs_params {
     int32_t com_fp64;   /* 1: node centres of mass from FP64 sums;
                            0: the reference's FP32 pairwise formula */
     int32_t walk_batch; /* nodes fetched per stack pop, 1..64 (0 = default 32) */
-    int32_t walk_blocks_per_sm; /* persistent walk occupancy (0 = default) */
+    int32_t walk_blocks_per_sm; /* blocks of 8 warps per SM of the walk, one
+                           warp a group (0 = default: all that fit, or, in
+                           contexts of few groups, two warps a group) */
     int32_t with_potential; /* 1: the walk also sums potentials (ACCEL .w) */
     int32_t tune_leaf_min;  /* gcs_autotune: smallest leaf size it may pick (0 = 1) */
     int32_t reserved[2];

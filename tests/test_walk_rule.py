@@ -1,0 +1,42 @@
+"""When a walk's groups get two warps each: the rule compiled for the host.  A
+caller's occupancy (walk_blocks_per_sm) always means the one-warp kernel."""
+import os
+import subprocess
+
+import pytest
+
+from conftest import PKG, ROOT
+
+SOURCE = """
+#include <cstdio>
+#include "gcs_internal.h"
+int main() {
+    int groups, sms, bps;
+    while (scanf("%d %d %d", &groups, &sms, &bps) == 3) printf("%d\\n", gcs::walk_pairs_pay(groups, sms, bps) ? 1 : 0);
+}
+"""
+
+CASES = [  # groups, SMs, blocks per SM -> two warps
+    (1, 148, 0, 1), (44, 148, 0, 1), (1408, 148, 0, 1), (100000, 148, 0, 0),
+    (1, 148, 1, 0), (44, 148, 4, 0), (1408, 148, 8, 0), (100000, 148, 2, 0),
+]
+
+
+@pytest.fixture(scope="module")
+def rule(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rule")
+    (d / "rule.cpp").write_text(SOURCE)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(PKG, "csrc"), "-I", os.path.join(ROOT, "include"), "-I",
+                    os.path.join(cuda, "include"), "-o", str(d / "rule"), str(d / "rule.cpp")], check=True)
+
+    def ask(*numbers):
+        out = subprocess.run([str(d / "rule")], input=" ".join(map(str, numbers)), capture_output=True, text=True,
+                             check=True).stdout
+        return int(out)
+    return ask
+
+
+@pytest.mark.parametrize("groups,sms,bps,two", CASES)
+def test_occupancy_means_one_warp(rule, groups, sms, bps, two):
+    assert rule(groups, sms, bps) == two
