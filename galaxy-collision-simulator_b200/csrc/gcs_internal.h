@@ -295,18 +295,31 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
                  int sm_count, unsigned long long* counts, int2* gstack, size_t gstack_entries,
                  cudaStream_t st, const WalkEpilogue& ep = WalkEpilogue(),
                  const WalkFrontier& fr = WalkFrontier());
-// Whether every group gets two warps: while all groups find a pair of warps
-// within two waves.  Walk stage in us, one warp a group / two (theta 0.5, leaf
-// 8, batch 64 from 16,384 on):
-//    1,408 particles  78 /  61       60,000 (0.7, leaf 4)     170 / 139
-//    8,192           170 / 121       75,000                   326 / 285
-//   16,384           199 / 135       110,000                  406 / 385
-//   45,056           309 / 225       131,072 (0.7, leaf 4)    289 / 295
-//   16 x 5,000       170 / 152       262,144                  737 / 770
+// Whether every group gets two warps.  A round's barriers of the two are paid
+// for by its nodes, so the line goes by the batch (both warps fetch nodes above
+// 32) and by theta (the fewer nodes, the shorter the rounds).  12 groups an SM
+// find their pair of warps resident at once; what is above takes a second
+// wave, which only long rounds pay for.  Walk stage in us, one warp a group /
+// two (leaf 8, 32-target groups; a theta of 1 with leaf 1):
+//   particles (groups an SM)  16,000 (3.4)   27,000-30,000 (6)  56,000 (12)  85,000 (18)
+//   batch 64, theta 0.5                         221 / 180       289 / 239    338 / 316
+//             theta 0.7                         133 / 113       161 / 139    187 / 185
+//             theta 1                            82 /  80       102 /  96    111 / 125
+//   batch 32, theta 0.5          187 / 161      240 / 219       309 / 291    366 / 397
+//             theta 0.7                         144 / 139       175 / 171    203 / 227
+//             theta 1             83 /  80       91 /  91       109 / 113    118 / 144
+//   batch 16, theta 0.5          236 / 218      282 / 281       399 / 408    476 / 554
+//             theta 1            106 / 109      116 / 123
+//   batch 8, theta 0.5           323 / 322      397 / 416       557 / 611    675 / 852
 // A caller's walk_blocks_per_sm is an occupancy of the one-warp kernel, so
 // setting it asks for that one.
-inline bool walk_pairs_pay(int n_groups, int sm_count, int blocks_per_sm) {
-    return blocks_per_sm <= 0 && n_groups <= 20 * sm_count;
+inline bool walk_pairs_pay(int n_groups, int sm_count, int blocks_per_sm, int batch, float theta2) {
+    const bool few_nodes = theta2 > 0.6f;  // (between 0.7 and 1)
+    const int per_sm = batch > 32    ? (few_nodes ? 12 : 20)
+                       : batch == 32 ? (few_nodes ? 6 : 12)
+                       : batch >= 16 ? (few_nodes ? 0 : 6)
+                                     : 0;
+    return blocks_per_sm <= 0 && per_sm > 0 && n_groups <= (int64_t)per_sm * sm_count;
 }
 int walk_max_blocks_per_sm(int batch, int with_potential, int targets_per_lane);
 // Persistent walk grid (blocks) for n_groups groups, and the global stack
