@@ -296,30 +296,33 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
                  cudaStream_t st, const WalkEpilogue& ep = WalkEpilogue(),
                  const WalkFrontier& fr = WalkFrontier());
 // Whether every group gets two warps.  A round's barriers of the two are paid
-// for by its nodes, so the line goes by the batch (both warps fetch nodes above
-// 32) and by theta (the fewer nodes, the shorter the rounds).  12 groups an SM
-// find their pair of warps resident at once; what is above takes a second
-// wave, which only long rounds pay for.  Walk stage in us, one warp a group /
-// two (leaf 8, 32-target groups; a theta of 1 with leaf 1):
-//   particles (groups an SM)  16,000 (3.4)   27,000-30,000 (6)  56,000 (12)  85,000 (18)
-//   batch 64, theta 0.5                         221 / 180       289 / 239    338 / 316
-//             theta 0.7                         133 / 113       161 / 139    187 / 185
-//             theta 1                            82 /  80       102 /  96    111 / 125
-//   batch 32, theta 0.5          187 / 161      240 / 219       309 / 291    366 / 397
-//             theta 0.7                         144 / 139       175 / 171    203 / 227
-//             theta 1             83 /  80       91 /  91       109 / 113    118 / 144
-//   batch 16, theta 0.5          236 / 218      282 / 281       399 / 408    476 / 554
-//             theta 1            106 / 109      116 / 123
-//   batch 8, theta 0.5           323 / 322      397 / 416       557 / 611    675 / 852
+// for by its terms: batch nodes (above 32 both warps fetch some) and up to
+// leaf_size sources of each opened one, so the line goes by their product.
+// Up to 12 groups an SM every group's pair of warps is resident at once; what
+// is above takes a second wave, which pays only for long rounds, and the longer
+// the fewer nodes a wide theta leaves (62,000 particles, 13 groups an SM, batch
+// 64, leaf 4: 1.08 at theta 0.5, 1.06 at 0.7, 0.90 at 1).  Walk stage, one warp's time over two
+// warps' (32-target groups; the one-warp time at batch 64, theta 0.5, leaf 4 is
+// 190 to 360 us):
+//   particles (groups an SM)         20,000 (4.2)  30,000 (6.3)  56,000 (12)  75,000 (16)
+//   batch 8   theta 0.5  leaf 4, 32  0.94, 1.12    0.92, 1.13    0.90, 1.11   0.75, 0.97
+//   batch 16  theta 0.5  leaf 4, 16  0.98, 1.13    0.94, 1.09    0.94, 1.06   0.78, 0.92
+//             theta 1    leaf 4, 16  0.98, 1.05    0.95, 1.01    0.93, 0.99   0.80, 0.90
+//   batch 32  theta 0.5  leaf 4, 16  1.03, 1.20    1.00, 1.17    1.00, 1.17   0.87, 1.03
+//             theta 1    leaf 4, 32  1.03, 1.19    0.99, 1.17    0.99, 1.12   0.84, 1.04
+//   batch 64  theta 0.5  leaf 1, 16  1.15, 1.33    1.11, 1.29    1.10, 1.27   1.00, 1.13
+//             theta 0.7  leaf 1, 16  1.13, 1.27    1.08, 1.24    1.10, 1.22   0.92, 1.07
+//             theta 1    leaf 1, 32  1.04, 1.22    1.03, 1.21    1.06, 1.18   0.83, 1.06
 // A caller's walk_blocks_per_sm is an occupancy of the one-warp kernel, so
 // setting it asks for that one.
-inline bool walk_pairs_pay(int n_groups, int sm_count, int blocks_per_sm, int batch, float theta2) {
-    const bool few_nodes = theta2 > 0.6f;  // (between 0.7 and 1)
-    const int per_sm = batch > 32    ? (few_nodes ? 12 : 20)
-                       : batch == 32 ? (few_nodes ? 6 : 12)
-                       : batch >= 16 ? (few_nodes ? 0 : 6)
-                                     : 0;
-    return blocks_per_sm <= 0 && per_sm > 0 && n_groups <= (int64_t)per_sm * sm_count;
+inline bool walk_pairs_pay(int n_groups, int sm_count, int blocks_per_sm, int batch, int leaf_size, float theta2) {
+    const int round = batch * leaf_size;
+    const float per_sm = round >= 256 && (float)round >= 2048.0f * theta2 ? 20.0f
+                         : batch > 32                                    ? 16.0f - 4.0f * theta2
+                         : round >= 256                                  ? 12.0f
+                         : round >= 128                                  ? 6.0f
+                                                                         : 0.0f;
+    return blocks_per_sm <= 0 && per_sm > 0.0f && (float)n_groups <= per_sm * (float)sm_count;
 }
 int walk_max_blocks_per_sm(int batch, int with_potential, int targets_per_lane);
 // Persistent walk grid (blocks) for n_groups groups, and the global stack

@@ -1803,7 +1803,7 @@ void launch_walk(const Layout& L, const WalkParams& wp, const float4* pos,
     // entries per warp region: the whole buffer split over this grid's warps
     const size_t units = gstack_entries / ((size_t)grid * kWalkWarps);
     const int cap = (int)(std::min<size_t>(units, (size_t)1 << 24) / (size_t)T);
-    if (T == 1 && !counts && walk_pairs_pay(n_groups, sm_count, blocks_per_sm, q.batch, q.theta2)) {
+    if (T == 1 && !counts && walk_pairs_pay(n_groups, sm_count, blocks_per_sm, q.batch, q.leaf_size, q.theta2)) {
         // two warps a group; the stack regions are shared out over the pairs
         const int64_t blocks = ((int64_t)n_groups + kPairBlockPairs - 1) / kPairBlockPairs;
         const int64_t pairs = blocks * kPairBlockPairs;
