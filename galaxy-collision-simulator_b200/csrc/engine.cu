@@ -422,11 +422,12 @@ int upload_groups(gcs_ctx* c) {
 }  // namespace
 
 // The process's pageable-copy threads, taken for one copy of `bytes` into
-// host; nullptr: copy plainly (pinned or small, or another thread has them).
+// host; nullptr: copy plainly (pinned or small, not worth them yet, or another
+// thread has them).
 static HostCopy* begin_host_copy(gcs_ctx* c, const void* host, size_t bytes) {
     if (bytes < HostCopy::kWorth || !is_pageable(host)) return nullptr;
     if (!c->host_copy) c->host_copy = HostCopy::acquire();
-    return c->host_copy && c->host_copy->begin() ? c->host_copy : nullptr;
+    return c->host_copy && c->host_copy->begin(bytes) ? c->host_copy : nullptr;
 }
 
 // Copy device memory to the caller's host memory on the context stream; the

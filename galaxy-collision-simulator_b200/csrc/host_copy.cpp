@@ -49,8 +49,29 @@ struct HostCopy::Impl {
     std::condition_variable cv;
     std::atomic<bool> active{false};
     bool stop = false;
-    const pid_t owner = getpid();         // the process that has the helpers
+    size_t plain = 0;                     // bytes copied plainly so far (owner's)
+    bool tried = false;                   // set_up has been called
+    pid_t owner = 0;                      // the process that has the helpers
     std::vector<std::thread> threads;
+
+    // The ring and the helpers; false: there is no pinned memory.
+    bool set_up() {
+        if (tried) return ring != nullptr;
+        tried = true;
+        owner = getpid();
+        for (auto& d : done) d.store(0, std::memory_order_relaxed);
+        if (cudaHostAlloc(reinterpret_cast<void**>(&ring), kPiece * kSlots, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            ring = nullptr;
+            return false;
+        }
+        try {
+            const int cores = (int)std::thread::hardware_concurrency();
+            for (int k = 0; k < std::min(kWorkers, cores - 1); ++k) threads.emplace_back([this] { help(); });
+        } catch (...) {  // fewer threads, or none: the caller's own still copies
+        }
+        return true;
+    }
 
     bool copy_one() {
         uint64_t i = claimed.load(std::memory_order_relaxed);
@@ -96,21 +117,9 @@ HostCopy::~HostCopy() { delete impl; }
 HostCopy* HostCopy::acquire() {
     std::lock_guard<std::mutex> lk(g_mu);
     if (!g_copy) {
-        const int cores = (int)std::thread::hardware_concurrency();
-        if (cores < 2) return nullptr;
+        if (std::thread::hardware_concurrency() < 2) return nullptr;
         Impl* im = new (std::nothrow) Impl();
         if (!im) return nullptr;
-        for (auto& d : im->done) d.store(0, std::memory_order_relaxed);
-        if (cudaHostAlloc(reinterpret_cast<void**>(&im->ring), kPiece * kSlots, cudaHostAllocPortable) != cudaSuccess) {
-            cudaGetLastError();
-            im->ring = nullptr;
-            delete im;
-            return nullptr;
-        }
-        try {
-            for (int k = 0; k < std::min(kWorkers, cores - 1); ++k) im->threads.emplace_back([im] { im->help(); });
-        } catch (...) {  // fewer threads, or none: the caller's own still copies
-        }
         g_copy = new (std::nothrow) HostCopy();
         if (!g_copy) {
             delete im;
@@ -133,12 +142,21 @@ void HostCopy::release() {
     }
     // a forked child has the object but not its threads: joining them would
     // wait for good, so there it is left to the end of the process
-    if (last && last->impl->owner == getpid()) delete last;
+    if (last && (!last->impl->tried || last->impl->owner == getpid())) delete last;
 }
 
-bool HostCopy::begin() {
+bool HostCopy::begin(size_t bytes) {
     Impl& m = *impl;
     if (!m.own.try_lock()) return false;
+    if (m.plain < kEarned) {
+        m.plain += std::min(bytes, kEarned);
+        m.own.unlock();
+        return false;
+    }
+    if (!m.set_up()) {
+        m.own.unlock();
+        return false;
+    }
     int dev = -1;
     bool ok = cudaGetDevice(&dev) == cudaSuccess;
     if (ok && dev != m.device) {  // events belong to a device

@@ -12,10 +12,12 @@
 // cost more than its walk), a 1920 x 1080 frame 799 -> 557 us.  Two, four and
 // eight threads copy 9.6 MB in 358, 264 and 423 us.
 //
-// One ring and its threads serve the process: made by the first context that
-// uses them, kept while such a context lives, given back with the last.  A
-// copy takes them for itself (begin() fails while another thread has them,
-// and callers then copy plainly).
+// One ring and its threads serve the process, kept while a context that copies
+// lives and given back with the last.  Making them takes 4 to 5 ms, which a
+// program with few copies does not get back (its first copy of 1 MiB took 5.1 ms
+// in place of 0.19, of 9.6 MB 5.0 in place of 0.8): copies go plainly until
+// kEarned bytes have, which has cost as much.  A copy takes the ring for itself
+// (begin() fails while another thread has it, and callers then copy plainly).
 #pragma once
 #include <cstddef>
 #include <cuda_runtime.h>
@@ -28,13 +30,14 @@ class HostCopy {
     static constexpr int kSlots = 8;
     static constexpr int kWorkers = 3;
     static constexpr size_t kWorth = 1 << 20;  // smaller copies go plainly
+    static constexpr size_t kEarned = 64 << 20;
 
-    // The process's instance, counted by user; nullptr where there is no
-    // pinned memory or no second core.
+    // The process's instance, counted by user; nullptr where there is no second
+    // core.
     static HostCopy* acquire();
     static void release();
 
-    bool begin();  // take it; false: busy
+    bool begin(size_t bytes);  // take it for a copy of bytes; false: copy plainly
     // Queue a copy of `bytes` from device memory on `st`; blocks (working on
     // landed pieces) while the ring is full.  Nothing is queued after an error.
     void add(void* dst, const void* src, size_t bytes, cudaStream_t st);
