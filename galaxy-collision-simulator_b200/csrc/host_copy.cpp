@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
@@ -42,12 +43,12 @@ struct HostCopy::Impl {
     std::atomic<uint64_t> landed{0};      // pieces whose device copy is done
     std::atomic<uint64_t> claimed{0};     // pieces taken by a copying thread
     std::atomic<uint64_t> done[kSlots];   // piece number + 1 last copied out of the slot
-    uint64_t queued = 0;                  // owner's
+    std::atomic<uint64_t> queued{0};      // pieces whose device copy is queued (the owner writes it)
     cudaError_t error = cudaSuccess;      // owner's
     std::mutex own;                       // the running copy
     std::mutex mu;                        // wakes the helpers
     std::condition_variable cv;
-    std::atomic<bool> active{false};
+    std::atomic<int> asleep{0};           // helpers that wait for a piece
     bool stop = false;
     size_t plain = 0;                     // bytes copied plainly so far (owner's)
     bool tried = false;                   // set_up has been called
@@ -82,17 +83,34 @@ struct HostCopy::Impl {
         done[s].store(i + 1, std::memory_order_release);
         return true;
     }
+    // A helper sleeps until pieces are queued, which wakes it while the first
+    // of them travels, and goes back to sleep kAwake after the last: the chunks
+    // of a host step can be far apart while the device walks.  (asleep and
+    // queued are sequentially consistent: either the helper sees the piece or
+    // wake() sees the helper.)
     void help() {
+        using Clock = std::chrono::steady_clock;
         for (;;) {
             {
                 std::unique_lock<std::mutex> lk(mu);
-                cv.wait(lk, [&] { return stop || active.load(std::memory_order_relaxed); });
+                ++asleep;
+                cv.wait(lk, [&] { return stop || claimed.load() < queued.load(); });
+                --asleep;
                 if (stop) return;
             }
-            while (active.load(std::memory_order_relaxed))
-                if (!copy_one()) relax();
+            for (Clock::time_point last = Clock::now(); Clock::now() - last < kAwake;) {
+                if (copy_one() || claimed.load(std::memory_order_relaxed) < queued.load(std::memory_order_relaxed))
+                    last = Clock::now();
+                for (int k = 0; k < 4; ++k) relax();
+            }
         }
     }
+    void wake() {
+        if (asleep.load() == 0) return;
+        { std::lock_guard<std::mutex> lk(mu); }
+        cv.notify_all();
+    }
+    static constexpr std::chrono::microseconds kAwake{15};
     void drop_events() {
         for (cudaEvent_t& e : landed_ev) {
             if (e) cudaEventDestroy(e);
@@ -173,13 +191,8 @@ bool HostCopy::begin(size_t bytes) {
     }
     // the counters go on from the last copy (a helper may still be looking at
     // them); pieces that an error kept from landing are numbered again
-    m.queued = m.landed.load(std::memory_order_relaxed);
+    m.queued.store(m.landed.load(std::memory_order_relaxed));
     m.error = cudaSuccess;
-    {
-        std::lock_guard<std::mutex> lk(m.mu);
-        m.active.store(true, std::memory_order_release);
-    }
-    m.cv.notify_all();
     return true;
 }
 
@@ -187,7 +200,7 @@ bool HostCopy::begin(size_t bytes) {
 void HostCopy::poll() {
     Impl& m = *impl;
     uint64_t i = m.landed.load(std::memory_order_relaxed);
-    while (i < m.queued && m.error == cudaSuccess) {
+    while (i < m.queued.load(std::memory_order_relaxed) && m.error == cudaSuccess) {
         const cudaError_t e = cudaEventQuery(m.landed_ev[i % kSlots]);
         if (e == cudaErrorNotReady) break;
         if (e != cudaSuccess) {
@@ -206,7 +219,7 @@ void HostCopy::work() {
 void HostCopy::add(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     Impl& m = *impl;
     for (size_t at = 0; at < bytes && m.error == cudaSuccess; at += kPiece) {
-        const uint64_t i = m.queued;
+        const uint64_t i = m.queued.load(std::memory_order_relaxed);
         const int s = (int)(i % kSlots);
         // the slot's last piece has been copied out
         while (i >= kSlots && m.done[s].load(std::memory_order_acquire) != i - kSlots + 1 && m.error == cudaSuccess)
@@ -221,7 +234,8 @@ void HostCopy::add(void* dst, const void* src, size_t bytes, cudaStream_t st) {
             m.error = e;
             return;
         }
-        m.queued = i + 1;
+        m.queued.store(i + 1);
+        m.wake();
         poll();
     }
 }
@@ -236,13 +250,14 @@ cudaError_t HostCopy::finish() {
             if (m.done[i % kSlots].load(std::memory_order_acquire) != i + 1) return false;
         return true;
     };
-    while (m.error == cudaSuccess && m.landed.load(std::memory_order_relaxed) < m.queued) work();
+    while (m.error == cudaSuccess && m.landed.load(std::memory_order_relaxed) < m.queued.load(std::memory_order_relaxed))
+        work();
     while (!copied()) work();
+    m.queued.store(m.landed.load(std::memory_order_relaxed));  // (less after an error)
     // after an error no device copy may still be on its way into the ring
     if (m.error != cudaSuccess)
         for (int s = 0; s < kSlots; ++s)
             if (m.landed_ev[s]) cudaEventSynchronize(m.landed_ev[s]);
-    m.active.store(false, std::memory_order_release);
     const cudaError_t e = m.error;
     m.own.unlock();
     return e;
