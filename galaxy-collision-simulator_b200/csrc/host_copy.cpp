@@ -12,6 +12,7 @@
 #include <thread>
 #include <vector>
 
+#include <csignal>
 #include <unistd.h>
 
 namespace gcs {
@@ -66,11 +67,17 @@ struct HostCopy::Impl {
             ring = nullptr;
             return false;
         }
+        // the process's signals stay with its own threads: helpers inherit this
+        // mask and take none
+        sigset_t every, before;
+        sigfillset(&every);
+        const bool masked = pthread_sigmask(SIG_SETMASK, &every, &before) == 0;
         try {
             const int cores = (int)std::thread::hardware_concurrency();
             for (int k = 0; k < std::min(kWorkers, cores - 1); ++k) threads.emplace_back([this] { help(); });
         } catch (...) {  // fewer threads, or none: the caller's own still copies
         }
+        if (masked) pthread_sigmask(SIG_SETMASK, &before, nullptr);
         return true;
     }
 

@@ -47,6 +47,28 @@ def test_set_up_once_earned(gcs_mod, n):
         assert _threads() <= before
 
 
+def _blocked(task):
+    with open(f"/proc/self/task/{task}/status") as f:
+        return int(next(line.split()[1] for line in f if line.startswith("SigBlk")), 16)
+
+
+def test_helpers_take_no_signals(gcs_mod):
+    """The caller's handlers run on the caller's threads only."""
+    import signal
+    gcs = gcs_mod
+    n = 21 * PIECE
+    with gcs.Context(n) as ctx:
+        ctx.upload(_stars(gcs, n, 1))
+        before, mask = _threads(), signal.pthread_sigmask(signal.SIG_BLOCK, [])
+        for _ in range(8):
+            ctx.download()
+        helpers = _threads() - before
+        assert helpers
+        for s in (signal.SIGINT, signal.SIGTERM, signal.SIGALRM, signal.SIGUSR1, signal.SIGCHLD):
+            assert all(_blocked(t) >> (s - 1) & 1 for t in helpers)
+        assert signal.pthread_sigmask(signal.SIG_BLOCK, []) == mask
+
+
 def test_host_steps_across_it(gcs_mod):
     """Host steps into pageable memory before, at and after the set-up: the same
     Stars as device steps."""
