@@ -72,7 +72,6 @@ struct gcs_ctx {
     // walk frontiers: super-groups of consecutive groups, their lists
     SuperGroup* supers = nullptr;
     int32_t* sg_list = nullptr;
-    int32_t* sg_src = nullptr;
     int4* sg_meta = nullptr;
     int n_supers = 0;
     size_t supers_cap = 0;
@@ -89,7 +88,6 @@ struct gcs_ctx {
     Chunk* chunks = nullptr;
     float2* seg_bounds = nullptr;
     Star* staging = nullptr;
-    PlaybackStar* pb_staging = nullptr;
     unsigned char* scratch = nullptr;
     size_t scratch_cap = 0;
     uint32_t* status = nullptr;
@@ -290,8 +288,8 @@ void free_all(gcs_ctx* c) {
     if (c->host_copy) HostCopy::release();
     void* ptrs[] = {c->pos[0], c->pos[1], c->vel[0], c->vel[1], c->acc, c->keys[0], c->keys[1],
                     c->idx[0], c->idx[1], c->tr, c->bd, c->wn, c->com64, c->leaf_parent, c->seg_off,
-                    c->seg_id, c->groups, c->supers, c->sg_list, c->sg_src, c->sg_meta, c->perm, c->chunks,
-                    c->seg_bounds, c->staging, c->pb_staging,
+                    c->seg_id, c->groups, c->supers, c->sg_list, c->sg_meta, c->perm, c->chunks,
+                    c->seg_bounds, c->staging,
                     c->scratch, c->status, c->diag, c->targets, c->direct_out, c->direct_sums, c->counts,
                     c->walk_stack, c->render_acc, c->render_rgba, c->star_chunk_done};
     for (void* p : ptrs)
@@ -376,6 +374,7 @@ int upload_groups(gcs_ctx* c) {
     // scenario stepped across devices as in the whole scenario.
     const int per = groups_per_super(c->group_width);
     const int64_t span = (int64_t)per * c->group_width;  // targets of a full super-group
+    int64_t src_at = 0;
     for (int s = 0; s < c->nseg; ++s) {
         const int64_t a = c->h_seg_off[s], e = c->h_seg_off[s + 1];
         int64_t cur = -1;  // first target of the current super-group
@@ -391,7 +390,8 @@ int upload_groups(gcs_ctx* c) {
                 sg.start = (int32_t)sg_first;
                 sg.count = (int32_t)std::min<int64_t>(span, e - sg_first);
                 sg.seg = s;
-                sg.pad = 0;
+                sg.src_at = (int32_t)src_at;
+                src_at += (super_src_cap((int32_t)(e - a)) + kSuperSrcUnit - 1) / kSuperSrcUnit;
                 supers.push_back(sg);
                 cur = sg_first;
             }
@@ -399,7 +399,8 @@ int upload_groups(gcs_ctx* c) {
             groups.push_back(w);
         }
     }
-    if (groups.size() > c->groups_cap || supers.size() > c->supers_cap) {
+    if (groups.size() > c->groups_cap || supers.size() > c->supers_cap ||
+        src_at * kSuperSrcUnit * (int64_t)sizeof(int32_t) > c->capacity * (int64_t)sizeof(double4)) {
         c->last_error = "group table capacity exceeded";
         return GCS_ERR_CAPACITY;
     }
@@ -420,6 +421,11 @@ int upload_groups(gcs_ctx* c) {
 }
 
 }  // namespace
+
+// Playback records are packed where Stars are on their way in and out of the
+// other calls, which all wait for their copies (a bake's frame is still being
+// copied while the next step runs, and gcs_step stages nothing).
+static PlaybackStar* playback_staging(gcs_ctx* c) { return reinterpret_cast<PlaybackStar*>(c->staging); }
 
 // The process's pageable-copy threads, taken for one copy of `bytes` into
 // host; nullptr: copy plainly (pinned or small, not worth them yet, or another
@@ -486,7 +492,8 @@ static int walk_stage(gcs_ctx* c, const gcs_params* p, const WalkEpilogue& ep) {
     fr.supers = c->walk_frontier ? c->supers : nullptr;
     fr.n_supers = c->n_supers;
     fr.list = c->sg_list;
-    fr.src = c->sg_src;
+    fr.src = reinterpret_cast<int32_t*>(c->com64);  // no sums are needed after the aggregation
+    if (fr.supers) c->relay_empty = false;
     fr.meta = c->sg_meta;
     fr.perm = partitioned(c) ? c->perm : nullptr;
     fr.split_levels = split_levels(c->group_width);
@@ -817,13 +824,11 @@ static int allocate_state(gcs_ctx* c) {
     if (!rc) rc |= dalloc(c, &c->supers, max_supers);
     static_assert(kSuperCap / kSuperTargets >= 3, "the aggregation's lists fit sg_list: 3 words a particle");
     if (!rc) rc |= dalloc(c, &c->sg_list, max_supers * (size_t)kSuperCap);
-    if (!rc) rc |= dalloc(c, &c->sg_src, max_supers * (size_t)kSuperSrcCap);
     if (!rc) rc |= dalloc(c, &c->sg_meta, max_supers);
     if (!rc) rc |= dalloc(c, &c->perm, N);
     if (!rc) rc |= dalloc(c, &c->chunks, max_chunks);
     if (!rc) rc |= dalloc(c, &c->seg_bounds, (size_t)max_segments);
     if (!rc) rc |= dalloc(c, &c->staging, N);
-    if (!rc) rc |= dalloc(c, &c->pb_staging, N);
     if (!rc) rc |= dalloc(c, &c->status, 1);
     if (!rc) rc |= dalloc(c, &c->diag, 8);
     if (!rc) rc |= dalloc(c, &c->counts, kCountWords);
@@ -1040,11 +1045,12 @@ int gcs_download_playback(gcs_ctx* c, PlaybackStar* host, int64_t offset, int64_
     if (!c || !host || offset < 0 || n < 0 || offset + n > c->n) return GCS_ERR_ARG;
     if (n == 0) return GCS_OK;
     cudaSetDevice(c->device);
-    launch_pack_playback(c->pos[c->cur] + offset, c->vel[c->cur] + offset, c->pb_staging + offset,
+    PlaybackStar* staging = playback_staging(c);
+    launch_pack_playback(c->pos[c->cur] + offset, c->vel[c->cur] + offset, staging + offset,
                          n, c->stream);
     int rc = check_launch(c, "pack_playback");
     if (rc) return rc;
-    return copy_to_host(c, host, c->pb_staging + offset, sizeof(PlaybackStar) * (size_t)n);
+    return copy_to_host(c, host, staging + offset, sizeof(PlaybackStar) * (size_t)n);
 }
 
 // Capture the full step twice, once from each ping-pong parity of the
@@ -1924,7 +1930,7 @@ extern "C" int gcs_bake(gcs_ctx* c, const gcs_params* p, int32_t frames, const c
             rc = GCS_ERR_CUDA;
             break;
         }
-        if (n > 0) launch_pack_playback(c->pos[c->cur], c->vel[c->cur], c->pb_staging, n, c->stream);
+        if (n > 0) launch_pack_playback(c->pos[c->cur], c->vel[c->cur], playback_staging(c), n, c->stream);
         if ((rc = check_launch(c, "bake pack")) || cudaEventRecord(packed[k & 1], c->stream) != cudaSuccess) {
             rc = rc ? rc : GCS_ERR_CUDA;
             break;
@@ -1936,7 +1942,7 @@ extern "C" int gcs_bake(gcs_ctx* c, const gcs_params* p, int32_t frames, const c
             if (W.error) break;
         }
         if (cudaStreamWaitEvent(copy, packed[k & 1], 0) != cudaSuccess ||
-            (n > 0 && cudaMemcpyAsync(host[k & 1], c->pb_staging, bytes, cudaMemcpyDeviceToHost, copy) != cudaSuccess) ||
+            (n > 0 && cudaMemcpyAsync(host[k & 1], playback_staging(c), bytes, cudaMemcpyDeviceToHost, copy) != cudaSuccess) ||
             cudaEventRecord(copied[k & 1], copy) != cudaSuccess) {
             rc = GCS_ERR_CUDA;
             break;

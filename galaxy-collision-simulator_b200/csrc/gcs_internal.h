@@ -8,7 +8,8 @@
 //   keys[2]  u64 Morton codes, idx[2] u32 positions (radix-sort ping-pong)
 //   nodes_tr BvhNodeTraverse[n_internal], nodes_bd BvhNodeBuild[n_internal],
 //   wn       WalkNode[n_internal] (walk records: com, G*mass, width^2, codes)
-//   com64    double4 [n_internal] FP64 mass-weighted position sums
+//   com64    double4 [n_internal] FP64 mass-weighted position sums; after the
+//            aggregation, the walk's source lists of super-groups
 //   leaf_parent i32[N]
 //   seg_off  i64[S+1], seg_id i32[N], groups int4[n_groups]
 //   scratch  zeroed once per step (sort histograms, tile counters, look-back,
@@ -266,13 +267,19 @@ struct SuperGroup {
     int32_t start;
     int32_t count;
     int32_t seg;
-    int32_t pad;
+    int32_t src_at;  // its source list starts at unit src_at of kSuperSrcUnit
 };
+// Source lists stand one behind the other in the array of the aggregation's
+// FP64 sums, which nothing reads after it: 32 bytes a particle, where lists of
+// super_src_cap words of at least 193 targets each, or one of a whole smaller
+// segment, take 25 (a segment of few particles: whole units of 8 words).
+constexpr int kSuperSrcUnit = 8;
+__host__ __device__ constexpr int super_src_cap(int seg_n) { return seg_n < kSuperSrcCap ? seg_n : kSuperSrcCap; }
 struct WalkFrontier {
     const SuperGroup* supers = nullptr;  // null: every group walks from its root
     int n_supers = 0;
     int32_t* list = nullptr;  // [n_supers][kSuperCap]
-    int32_t* src = nullptr;   // [n_supers][kSuperSrcCap] sorted particle indices
+    int32_t* src = nullptr;   // sorted particle indices, per super-group from src_at on
     int4* meta = nullptr;     // per super-group: n_take, n_src, n_front, valid
     // Targets in group order (null: Morton order).  A full super-group of
     // kSuperTargets targets is split into its groups by recursive median

@@ -299,7 +299,7 @@ void launch_tiles(const Layout& L, int pass, int tiles, const uint64_t* keys_in,
 size_t pass_words(int64_t n) {
     const int tile = sort_tile(n);
     const int64_t tiles = n > 0 ? (n + tile - 1) / tile : 1;
-    return (size_t)(tiles + (tiles + kLookGroup - 1) / kLookGroup) * kRadix;
+    return (size_t)(tiles + tiles / kLookGroup) * kRadix;  // (only whole groups publish a sum)
 }
 
 }  // namespace
@@ -308,7 +308,7 @@ size_t sort_lookback_words(int64_t n, int passes) { return pass_words(n) * passe
 
 size_t sort_lookback_words_upto(int64_t n, int passes) {
     // one wave of tiles at most while the tile grows with n, then n / kSortTile
-    const size_t wave = (size_t)(kSortWave + (kSortWave + kLookGroup - 1) / kLookGroup) * kRadix;
+    const size_t wave = (size_t)(kSortWave + kSortWave / kLookGroup) * kRadix;
     return std::max(pass_words(n), n > kSortSmallMax ? wave : pass_words(std::min(n, kSortSmallMax))) * passes;
 }
 

@@ -510,7 +510,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                     WC.all_take += (uint32_t)fm.x;
                     WC.r_list += (uint32_t)fm.x;
                 }
-                const int32_t* sl = fr.src + (size_t)grp.super * kSuperSrcCap;
+                const int32_t* sl = fr.src + (size_t)__ldg(&fr.supers[grp.super].src_at) * kSuperSrcUnit;
                 for (int base = 0; base < fm.y; base += kSrcCap) {
                     const int cnt = min(kSrcCap, fm.y - base);
                     for (int e = lane; e < cnt; e += 32) {
@@ -1113,7 +1113,7 @@ walk_pair_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos, const 
                         half_add<kPot>(A, d, zm, true, true);
                     }
                 }
-                const int32_t* sl = fr.src + (size_t)grp.super * kSuperSrcCap;
+                const int32_t* sl = fr.src + (size_t)__ldg(&fr.supers[grp.super].src_at) * kSuperSrcUnit;
                 for (int base = 0; base < fm.y; base += kSrcCap) {
                     const int cnt = min(kSrcCap, fm.y - base);
                     for (int e = lane + 32 * w; e < cnt; e += 64) {
@@ -1532,7 +1532,8 @@ frontier_kernel(Layout L, const float4* __restrict__ pos, const WalkNode* __rest
     const int off = (int)__ldg(L.seg_off + s);
     const int seg_n = (int)__ldg(L.seg_off + s + 1) - off;
     int32_t* list = fr.list + (size_t)sgi * kSuperCap;
-    int32_t* src = fr.src + (size_t)sgi * kSuperSrcCap;
+    int32_t* src = fr.src + (size_t)sg.src_at * kSuperSrcUnit;
+    const int src_cap = super_src_cap(seg_n);
     int n_take = 0, n_src = 0, n_front = 0;
     bool ok = true;
     if (seg_n >= 2) {
@@ -1594,7 +1595,7 @@ frontier_kernel(Layout L, const float4* __restrict__ pos, const WalkNode* __rest
             const uint32_t excl = incl - both;
             const uint32_t total = __shfl_sync(kFull, incl, 31);
             const int push_total = (int)(total >> 16), src_total = (int)(total & 0xFFFFu);
-            if (n_take + n_front + add_take + add_front > kSuperCap || n_src + src_total > kSuperSrcCap ||
+            if (n_take + n_front + add_take + add_front > kSuperCap || n_src + src_total > src_cap ||
                 top + push_total > kFrontStack) {
                 ok = false;
                 break;

@@ -50,7 +50,7 @@ constexpr size_t kStaticTiles = kSortWave;
 static_assert((kStaticSortMax + sort_tile(kStaticSortMax) - 1) / sort_tile(kStaticSortMax) <= kSortWave &&
                   kSortSmallMax / kSortSmallTile <= kSortWave,
               "every call's tiles fit the array");
-constexpr size_t kStaticSlots = kStaticTiles + (kStaticTiles + kLookGroup - 1) / kLookGroup;
+constexpr size_t kStaticSlots = kStaticTiles + kStaticTiles / kLookGroup;
 constexpr size_t kLookbackWords = kStaticSlots * kRadix * kKeyPasses;
 constexpr size_t kScratchWords = kHistWords + kTicketWords + kStatusWords + kLookbackWords;
 
