@@ -1010,9 +1010,9 @@ def main():
                 "walk_stack_peak": stack_peak, "walk_stack_global_per_warp": stack_global,
                 "walk_lane_use": lane_use}
     passes = 8
-    # bounds + decode, encode, the sort passes, gather, build, aggregate,
+    # bounds + decode, encode, the sort passes, gather, build, aggregate + rise,
     # partition, frontier, walk (which also applies the kick/drift)
-    launches_per_step = 2 + 1 + passes + 1 + 1 + 1 + 3
+    launches_per_step = 2 + 1 + passes + 1 + 1 + 2 + 3
     line = {"metric": "particle-steps/s", "value": value, "unit": "particle-steps/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": t_max / args.steps,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",

@@ -49,11 +49,14 @@ constexpr int kMaxPasses = 10;         // + up to two segment-id digits
 // Keys per sort tile by the number of pairs (sort_tile): up to kSortSmallMax
 // pairs, one 1024-key tile of 256 threads per SM; above, 512 threads with
 // the fewest keys each (2 to 8) that let all tiles be resident at once, two
-// to an SM, so that a pass is one wave of equal tiles.  Eight passes in CUDA
-// events, 4,096-key tiles for every size before / this rule now: 1,408 pairs
-// 71.7 / 54.2 us, 45,056 91.2 / 70.8, 300,000 104.5 / 89.2, 777,777 150.6 /
-// 124.0, 1,048,576 153.2 / 138.4 (a fixed 4,096-key tile with the new
-// look-back: 777,777 140.3, 1,048,576 140.4).
+// to an SM, so that a pass is one wave of equal tiles.  (B200's 148 SMs, as
+// constants: the static sort's array is sized by them.  Any SM count sorts.)
+// The sort stage in us, CUDA events around it alone, plain launches: 4,096-key
+// tiles for every size and a one-level look-back / now: 1,408 pairs 76.5 / 45.5,
+// 45,056 90.1 / 57.3, 300,000 103.4 / 68.7, 777,777 150.7 / 104.4, 1,048,576
+// 154.6 / 113.6.  The rule's own part, before launches overlapped: 4,096-key
+// tiles with the two-level look-back 140.3 at 777,777 and 140.4 at 1,048,576,
+// this rule 124.0 and 138.4.
 constexpr int kSortWave = 2 * 148;
 constexpr int kSortSmallTile = 1024;
 constexpr int64_t kSortSmallMax = 148 * 1024;
@@ -125,12 +128,14 @@ void launch_encode(const Layout& L, const float4* pos, int bounds_mode, float gm
 // Bounds, encode and sort of one segment of up to kFrontMax particles in one
 // launch (k_front.cu): the sorted keys and positions.  front_available: the
 // current device runs its clusters.
-// Whole step in us, separate stages / one launch, plain launches and graph:
-//    1,408 particles  188 / 136  and 154 / 123
-//    8,192            228 / 176      194 / 168
-//   32,768            321 / 287      290 / 281
-//   45,056            354 / 324      320 / 317
-//   65,536            413 / 400      380 / 392
+// Whole step in us (theta 0.5, leaf 8), separate stages / one launch, plain
+// launches and graph:
+//    1,408 particles  140 / 116  and 130 / 111
+//    8,192            210 / 187      202 / 186
+//   16,384            252 / 232      241 / 228
+//   32,768            310 / 298      302 / 294
+//   45,056            350 / 347      338 / 342
+//   49,152            355 / 355      346 / 350
 constexpr int kFrontMax = 49152;
 constexpr int kFrontBoundsReduce = 0;  // reduce the bounds, and write seg_bounds
 constexpr int kFrontBoundsGiven = 1;   // read seg_bounds

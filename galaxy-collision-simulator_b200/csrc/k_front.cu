@@ -1,16 +1,17 @@
 // k_front.cu - bounds, Morton encode and radix sort of a small scenario in
 // one launch: one thread-block cluster holds all keys in shared memory.
 //
-// The three stages of up to kFrontMax particles of one segment were eleven
-// launches, each as long as its latency chain (bounds and encode 10 us each,
-// eight sort passes of 7 to 9 us; 78, 80 and 93 us at 1,000, 8,192 and 49,152
-// particles, 26, 34 and 67 us now; 1,024 threads a block 33, 39 and 70 us).  Here a cluster of 8 or 16 blocks keeps
-// every (key, position) pair in its shared memory for all eight passes of the
-// same stable LSD sort (k_sort.cu): a block ranks its own pairs with warp
-// ballots and puts them in digit order, the blocks exchange digit counts
-// through distributed shared memory, and each run of a digit moves to its
-// place in the block that owns it in the next pass.  Two cluster barriers a pass; nothing but the particles,
-// the sorted keys and the positions touches global memory.
+// The three stages of up to kFrontMax particles of one segment are eleven
+// launches on their own, each as long as its latency chain: together 56, 62, 63
+// and 64 us at 1,408, 8,192, 32,768 and 49,152 particles (CUDA events, plain
+// launches), 29, 37, 54 and 66 in one (1,024 threads a block took 3 to 7 us
+// more).  Here a cluster of 8 or 16 blocks keeps every (key, position) pair in
+// its shared memory for all eight passes of the same stable LSD sort
+// (k_sort.cu): a block ranks its own pairs with warp ballots and puts them in
+// digit order, the blocks exchange digit counts through distributed shared
+// memory, and each run of a digit moves to its place in the block that owns it
+// in the next pass.  Two cluster barriers a pass; nothing but the particles, the
+// sorted keys and the positions touches global memory.
 //
 // Keys, order and bounds are bit for bit those of the separate stages.
 #include <algorithm>

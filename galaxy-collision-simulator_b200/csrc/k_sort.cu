@@ -37,9 +37,10 @@
 //    runs of equal digits.
 //
 // A pass is bound by the latency of one tile (launch, ticket, loads, ranking,
-// look-back, write-out), not by bytes: 17.3 us a pass at 1,048,576 pairs
-// (25 MB, 1.45 TB/s; 19.2 us before the two-level look-back), 8.8 us at 45,056
-// (11.4 before).
+// look-back, write-out), not by bytes.  An eighth of the sort stage (CUDA events
+// around it alone, plain launches, two memsets included): 14.2 us at 1,048,576
+// pairs (25 MB, 1.8 TB/s), 7.2 at 45,056; 19.3 and 11.3 with the one-level
+// look-back and launches that do not overlap (pdl.cuh).
 //
 // With more than one segment, one or two further stable passes order by the
 // segment id of each element's source position; the result is every segment
@@ -317,8 +318,9 @@ void launch_sort_pass(const Layout& L, int pass, const uint64_t* keys_in, const 
                       uint32_t* tile_counter, uint32_t* lookback, uint32_t* status,
                       cudaStream_t st) {
     if (L.n <= 0) return;
-    // every tile size at the first call on a device, so that a later call of
-    // another size may be its first within a stream capture
+    // every tile size at the first call on a device, which may be a captured one
+    // (the attribute is set at once, not on the stream): no call after it sets
+    // anything
     static std::once_flag configured[kMaxDevices];
     once_per_device(configured, [] {
         configure_tiles<256, kSortSmallTile / 256>();

@@ -824,7 +824,7 @@ walk_kernel(Layout L, WalkParams wp, const float4* __restrict__ pos,
                                                    : ((r == 0 && e.y < 0) ? ~e.y : ~e.z);
                                 const int at = nsrc + (j - base);
                                 W.srcp[at] = particle;
-    #pragma unroll
+#pragma unroll
                                 for (int t = 0; t < T; ++t)
                                     W.srcm[t][at] = reinterpret_cast<const uint32_t*>(W.pmask[t])[lo];
                             }
