@@ -66,7 +66,7 @@ typedef struct BvhNodeTraverse {
 typedef struct BvhNodeBuild {
     float min_x, min_y, min_z;
     float max_x, max_y, max_z;
-    int32_t flag;       /* arrival counter of the bottom-up pass */
+    int32_t flag;       /* reference: arrival counter of the bottom-up pass; here 0 */
     int32_t parent;     /* -1 at a segment root */
 } BvhNodeBuild;
 
