@@ -2,6 +2,7 @@
 for the first copies (a program with few would wait longer for them than for
 its copies), once 64 MiB have been copied plainly, and given back with the last
 context that copied.  Copies on both sides of that, and across it, are right."""
+import gc
 import os
 
 import numpy as np
@@ -28,6 +29,7 @@ def _stars(gcs, n, seed):
 def test_set_up_once_earned(gcs_mod, n):
     gcs = gcs_mod
     assert os.cpu_count() >= 2
+    gc.collect()  # no context of another test is still to go
     st = _stars(gcs, n, 1)
     for _ in range(2):
         with gcs.Context(n) as ctx:
@@ -36,7 +38,7 @@ def test_set_up_once_earned(gcs_mod, n):
             plain = -(-(64 << 20) // (32 * n))  # downloads that make 64 MiB
             for k in range(plain):
                 assert ctx.download().tobytes() == st.tobytes()
-                assert _threads() == before, k
+                assert not _threads() - before, k
             for _ in range(3):
                 assert ctx.download().tobytes() == st.tobytes()
             assert 1 <= len(_threads() - before) <= 3
@@ -57,6 +59,7 @@ def test_helpers_take_no_signals(gcs_mod):
     import signal
     gcs = gcs_mod
     n = 21 * PIECE
+    gc.collect()
     with gcs.Context(n) as ctx:
         ctx.upload(_stars(gcs, n, 1))
         before, mask = _threads(), signal.pthread_sigmask(signal.SIG_BLOCK, [])
