@@ -44,12 +44,13 @@ struct HostCopy::Impl {
     std::atomic<uint64_t> landed{0};      // pieces whose device copy is done
     std::atomic<uint64_t> claimed{0};     // pieces taken by a copying thread
     std::atomic<uint64_t> done[kSlots];   // piece number + 1 last copied out of the slot
-    std::atomic<uint64_t> queued{0};      // pieces whose device copy is queued (the owner writes it)
+    uint64_t queued = 0;                  // owner's
     cudaError_t error = cudaSuccess;      // owner's
     std::mutex own;                       // the running copy
     std::mutex mu;                        // wakes the helpers
     std::condition_variable cv;
-    std::atomic<int> asleep{0};           // helpers that wait for a piece
+    std::atomic<int> asleep{0};           // helpers that wait for a call
+    std::atomic<uint64_t> calls{0};
     bool stop = false;
     size_t plain = 0;                     // bytes copied plainly so far (owner's)
     bool tried = false;                   // set_up has been called
@@ -90,34 +91,37 @@ struct HostCopy::Impl {
         done[s].store(i + 1, std::memory_order_release);
         return true;
     }
-    // A helper sleeps until pieces are queued, which wakes it while the first
-    // of them travels, and goes back to sleep kAwake after the last: the chunks
-    // of a host step can be far apart while the device walks.  (asleep and
-    // queued are sequentially consistent: either the helper sees the piece or
-    // wake() sees the helper.)
+    // A helper sleeps until it is called: when a piece is queued, so that it
+    // wakes while the piece travels, and when one has landed (its copy may have
+    // been queued behind a long step).  It goes back to sleep when no piece has
+    // landed for kFirst after a call or kAwake after its last one: the chunks of
+    // a host step can be far apart while the device walks.  (asleep and calls
+    // are sequentially consistent: either the helper sees the call or wake()
+    // sees the helper.)
     void help() {
         using Clock = std::chrono::steady_clock;
-        for (;;) {
+        for (uint64_t seen = 0;;) {
             {
                 std::unique_lock<std::mutex> lk(mu);
                 ++asleep;
-                cv.wait(lk, [&] { return stop || claimed.load() < queued.load(); });
+                cv.wait(lk, [&] { return stop || calls.load() != seen; });
                 --asleep;
                 if (stop) return;
             }
-            for (Clock::time_point last = Clock::now(); Clock::now() - last < kAwake;) {
-                if (copy_one() || claimed.load(std::memory_order_relaxed) < queued.load(std::memory_order_relaxed))
-                    last = Clock::now();
-                for (int k = 0; k < 4; ++k) relax();
+            for (Clock::time_point until = Clock::now() + kFirst; Clock::now() < until;) {
+                if (copy_one()) until = Clock::now() + kAwake;
+                else for (int k = 0; k < 4; ++k) relax();
+                seen = calls.load();  // calls while awake need no other turn
             }
         }
     }
     void wake() {
+        ++calls;
         if (asleep.load() == 0) return;
         { std::lock_guard<std::mutex> lk(mu); }
         cv.notify_all();
     }
-    static constexpr std::chrono::microseconds kAwake{15};
+    static constexpr std::chrono::microseconds kFirst{50}, kAwake{15};
     void drop_events() {
         for (cudaEvent_t& e : landed_ev) {
             if (e) cudaEventDestroy(e);
@@ -198,7 +202,7 @@ bool HostCopy::begin(size_t bytes) {
     }
     // the counters go on from the last copy (a helper may still be looking at
     // them); pieces that an error kept from landing are numbered again
-    m.queued.store(m.landed.load(std::memory_order_relaxed));
+    m.queued = m.landed.load(std::memory_order_relaxed);
     m.error = cudaSuccess;
     return true;
 }
@@ -206,8 +210,9 @@ bool HostCopy::begin(size_t bytes) {
 // Take note of pieces that have landed (in order).
 void HostCopy::poll() {
     Impl& m = *impl;
-    uint64_t i = m.landed.load(std::memory_order_relaxed);
-    while (i < m.queued.load(std::memory_order_relaxed) && m.error == cudaSuccess) {
+    const uint64_t before = m.landed.load(std::memory_order_relaxed);
+    uint64_t i = before;
+    while (i < m.queued && m.error == cudaSuccess) {
         const cudaError_t e = cudaEventQuery(m.landed_ev[i % kSlots]);
         if (e == cudaErrorNotReady) break;
         if (e != cudaSuccess) {
@@ -216,6 +221,7 @@ void HostCopy::poll() {
         }
         m.landed.store(++i, std::memory_order_release);
     }
+    if (i > before) m.wake();
 }
 
 void HostCopy::work() {
@@ -226,7 +232,7 @@ void HostCopy::work() {
 void HostCopy::add(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     Impl& m = *impl;
     for (size_t at = 0; at < bytes && m.error == cudaSuccess; at += kPiece) {
-        const uint64_t i = m.queued.load(std::memory_order_relaxed);
+        const uint64_t i = m.queued;
         const int s = (int)(i % kSlots);
         // the slot's last piece has been copied out
         while (i >= kSlots && m.done[s].load(std::memory_order_acquire) != i - kSlots + 1 && m.error == cudaSuccess)
@@ -241,7 +247,7 @@ void HostCopy::add(void* dst, const void* src, size_t bytes, cudaStream_t st) {
             m.error = e;
             return;
         }
-        m.queued.store(i + 1);
+        m.queued = i + 1;
         m.wake();
         poll();
     }
@@ -257,10 +263,8 @@ cudaError_t HostCopy::finish() {
             if (m.done[i % kSlots].load(std::memory_order_acquire) != i + 1) return false;
         return true;
     };
-    while (m.error == cudaSuccess && m.landed.load(std::memory_order_relaxed) < m.queued.load(std::memory_order_relaxed))
-        work();
+    while (m.error == cudaSuccess && m.landed.load(std::memory_order_relaxed) < m.queued) work();
     while (!copied()) work();
-    m.queued.store(m.landed.load(std::memory_order_relaxed));  // (less after an error)
     // after an error no device copy may still be on its way into the ring
     if (m.error != cudaSuccess)
         for (int s = 0; s < kSlots; ++s)

@@ -10,11 +10,12 @@
 // with 16 cores: 9.6 MB of Stars 638 -> 340 us, a host step of 300,000
 // particles into pageable memory 1,529 -> 651 us (its 64 plain chunk copies
 // cost more than its walk), a 1920 x 1080 frame 799 -> 557 us.  Two, four and
-// eight threads copy 9.6 MB in 358, 264 and 423 us.  The helpers are awake while
-// pieces are queued and sleep between the chunks of a long walk (CPU time of a
-// host step of 1,000,000 particles at theta 0.5, 3.07 ms: 8.6 ms with helpers
-// awake from the first chunk to the last, 6.8 so; woken by a piece that has
-// landed instead, 5.2, but a host step of 300,000 took 0.65 in place of 0.60).
+// eight threads copy 9.6 MB in 358, 264 and 423 us.  The helpers are
+// called when a piece is queued and when one has landed, and sleep behind queued
+// steps and between the chunks of a long walk (CPU time of a host step of
+// 1,000,000 particles at theta 0.5, 3.06 ms: 8.6 ms with helpers awake from the
+// first chunk to the last, 6.6 so; called by landed pieces alone, 5.2, but a host
+// step of 300,000 took 0.65 ms in place of 0.60).
 //
 // One ring and its threads serve the process, kept while a context that copies
 // lives and given back with the last.  Making them takes 4 to 5 ms, which a

@@ -196,7 +196,7 @@ int32_t gcs_graph_builds(const gcs_ctx* ctx);
  * downloads and gcs_render_frame) go through 4 MiB of pinned memory and up to
  * three helper threads that the process shares: made once its living contexts
  * have copied 64 MiB plainly, given back with the last of them, and busy only
- * while pieces are on their way; a copy that finds them taken by another
+ * while pieces arrive; a copy that finds them taken by another
  * thread goes plainly.  The Stars and the device state are the same bits as
  * gcs_run_stages(bounds..integrate) followed by gcs_download_stars. */
 int gcs_step_host(gcs_ctx* ctx, const gcs_params* p, Star* host);
